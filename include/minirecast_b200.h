@@ -169,6 +169,14 @@ int mr_backproject_staged(const mr_ring* ring, const mr_view* views_dev,
                           const mr_grid* grids_dev, const mr_tile* tiles_dev, int64_t n_tiles,
                           float* out_dev, int32_t* status_dev, void* stream);
 
+/* The same sum over one regular grid (no flags) that is deep along i, j and k: a volume,
+ * in blocks of 16 x 16 x 16 voxels whose footprints are staged once per view. Views whose
+ * detector column and depth do not change along j (the volume's z on the usual orbit) share
+ * their reciprocal, column and horizontal weight along each column of a block. The grid
+ * record is read on the host and passed by value. Ring and status as above. */
+int mr_backproject_volume(const mr_ring* ring, const mr_view* views_dev, const mr_grid* grid_host,
+                          float* out_dev, int32_t* status_dev, void* stream);
+
 /* Persistent form of mr_backproject_staged for serving: a fixed grid of CTA clusters
  * (as many as fit on the GPU at once, at most max_tiles) pulls tile indices from a work
  * counter until it reaches min(*n_tiles_dev, max_tiles) (device int64; max_tiles <= 2^31),

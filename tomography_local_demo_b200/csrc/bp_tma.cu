@@ -16,14 +16,9 @@
 //     rare footprints larger than a stage fall back to predicated global loads.
 // Each warp covers compact 8 (j) x 4 (i) sample patches so its LDS gathers touch a small
 // 2D patch (few bank conflicts) for any plane orientation.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include <cooperative_groups.h>
-#include <mutex>
-#include <type_traits>
 
-#include "mr_common.cuh"
+#include "bp_stage.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -34,12 +29,7 @@ constexpr int ST_CONSUMERS = 8;               // consumer warps (one 32 x 32 til
 constexpr int ST_THREADS = 32 * (ST_CONSUMERS + 1);   // + one producer warp
 constexpr int ST_PPT = 4;                     // samples per consumer thread (rows i, i+2, i+4, i+6)
 constexpr int ST_DI = 2;                      // row step between a thread's samples
-constexpr int ST_BOX_H = 8;                   // rows per TMA box
 constexpr int ST_CLUSTER = 4;                 // CTAs per tile, each a quarter of the views
-constexpr float MAGIC = 12582912.0f;          // 1.5 * 2^23
-constexpr int MAGIC_BITS = 0x4B400000;
-#define kMagic2 make_float2(MAGIC, MAGIC)
-#define kNeg2 make_float2(-1.f, -1.f)
 
 template <typename T> struct StageGeom;
 // Row widths (elements) are 16-byte multiples whose word pitch shifts successive rows
@@ -50,7 +40,6 @@ template <> struct StageGeom<__nv_bfloat16> { static constexpr int W = 88, ALIGN
 template <> struct StageGeom<__half> { static constexpr int W = 88, ALIGN = 8, STAGES = 4, MAXB = 10; };
 template <> struct StageGeom<float> { static constexpr int W = 84, ALIGN = 4, STAGES = 3, MAXB = 8; };
 
-enum : int { MODE_STAGED = 0, MODE_GLOBAL = 1, MODE_SKIP = 2 };
 
 // What the consumer warps read per (tile, view): the local affine maps of the projective
 // numerators u, v and denominator w, (value at the tile origin, d/di, d/dj), in stage-local
@@ -64,103 +53,6 @@ struct __align__(16) ViewMeta {
     ViewRec rec;
     int x0, r0, nbox, mode;
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait: gives up after `limit` polls and reports it (never spins forever).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status) {
-    for (int it = 0; it < (1 << 22); ++it)
-        if (mbar_try_wait(bar, parity)) return true;
-    if (status) atomicExch(status, MR_ERR_TIMEOUT);
-    return false;
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
-                                            uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
-}
-
-__device__ __forceinline__ unsigned short lds_u16(uint32_t addr) {
-    unsigned short u;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(u) : "r"(addr));
-    return u;
-}
-// a - c, rounded to nearest, for a 16-bit value a (raw BF16 / FP16 bits) and an FP32 c
-template <typename T>
-__device__ __forceinline__ float sub16_f32(unsigned short a, float c) {
-    float d;
-    if constexpr (std::is_same<T, __nv_bfloat16>::value)
-        asm("sub.rn.f32.bf16 %0, %1, %2;" : "=f"(d) : "h"(a), "f"(c));
-    else
-        asm("sub.rn.f32.f16 %0, %1, %2;" : "=f"(d) : "h"(a), "f"(c));
-    return d;
-}
-
-template <typename T>
-__device__ __forceinline__ float lds_elem(uint32_t addr);
-template <>
-__device__ __forceinline__ float lds_elem<float>(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-    return v;
-}
-template <>
-__device__ __forceinline__ float lds_elem<__nv_bfloat16>(uint32_t addr) {
-    unsigned short u;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(u) : "r"(addr));
-    return __uint_as_float(static_cast<uint32_t>(u) << 16);
-}
-template <>
-__device__ __forceinline__ float lds_elem<__half>(uint32_t addr) {
-    unsigned short u;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(u) : "r"(addr));
-    return __half2float(__ushort_as_half(u));
-}
-
-// Global-memory bilinear (fallback for footprints larger than a stage).
-template <typename T>
-__device__ __forceinline__ float bilerp_global(const T* __restrict__ q, int R, int C, int pitch,
-                                               float row, float col) {
-    row = fminf(fmaxf(row, -2.f), (float)R + 1.f);
-    col = fminf(fmaxf(col, -2.f), (float)C + 1.f);
-    const float r0f = floorf(row), c0f = floorf(col);
-    const float fr = row - r0f, fc = col - c0f;
-    const int r0 = (int)r0f, c0 = (int)c0f;
-    const bool rin0 = (unsigned)r0 < (unsigned)R, rin1 = (unsigned)(r0 + 1) < (unsigned)R;
-    const bool cin0 = (unsigned)c0 < (unsigned)C, cin1 = (unsigned)(c0 + 1) < (unsigned)C;
-    const T* p = q + (ptrdiff_t)r0 * pitch + c0;
-    const float q00 = (rin0 && cin0) ? ld_elem(p) : 0.f;
-    const float q01 = (rin0 && cin1) ? ld_elem(p + 1) : 0.f;
-    const float q10 = (rin1 && cin0) ? ld_elem(p + pitch) : 0.f;
-    const float q11 = (rin1 && cin1) ? ld_elem(p + pitch + 1) : 0.f;
-    const float a = fmaf(fc, q01 - q00, q00);
-    const float b = fmaf(fc, q11 - q10, q10);
-    return fmaf(fr, b - a, a);
-}
 
 __device__ __forceinline__ bool in_box_fp64_t(const mr_grid& g, int i, int j) {
     const double aj = __dmul_rn((double)j - g.mask_half, g.mask_delta);
@@ -521,43 +413,12 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__
 }
 
 // ---------------------------------------------------------------- host side
-static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    });
-    return fn;
-}
-
-template <typename T>
-static int make_ring_map(const mr_ring* ring, CUtensorMap* map) {
-    auto fn = encode_fn();
-    if (!fn) return MR_ERR_CUDA;
-    const CUtensorMapDataType dt = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                                   : (std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                                                     : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
-    const cuuint64_t dims[3] = {(cuuint64_t)ring->cols, (cuuint64_t)ring->rows, (cuuint64_t)ring->n_slots};
-    const cuuint64_t strides[2] = {(cuuint64_t)ring->col_pitch * sizeof(T),
-                                   (cuuint64_t)ring->slot_stride * sizeof(T)};
-    const cuuint32_t box[3] = {(cuuint32_t)StageGeom<T>::W, (cuuint32_t)ST_BOX_H, 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, dt, 3, ring->data, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? MR_OK : MR_ERR_INVALID;
-}
-
 template <int KIND, typename T>
 static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
                          const mr_tile* tiles, int64_t n_tiles, float* out, int* status, cudaStream_t st,
                          const int64_t* n_tiles_dev = nullptr, unsigned int* counter = nullptr) {
     CUtensorMap map;
-    int rc = make_ring_map<T>(ring, &map);
+    int rc = make_ring_map<T>(ring, StageGeom<T>::W, &map);
     if (rc != MR_OK) return rc;
     constexpr int S = StageGeom<T>::STAGES;
     const size_t smem = (size_t)S * StageGeom<T>::W * ST_BOX_H * StageGeom<T>::MAXB * sizeof(T) +
@@ -600,19 +461,6 @@ static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_gri
         }
     }
     MR_CUDA_TRY(cudaGetLastError());
-    return MR_OK;
-}
-
-static int check_staged_ring(const mr_ring* ring) {
-    if (!ring || !ring->data) return MR_ERR_INVALID;
-    if (ring->rows <= 0 || ring->cols <= 0 || ring->col_pitch < ring->cols || ring->n_slots <= 0)
-        return MR_ERR_INVALID;
-    if (ring->slot_stride < (int64_t)ring->rows * ring->col_pitch) return MR_ERR_INVALID;
-    if (ring->kind != MR_CONE && ring->kind != MR_PARALLEL) return MR_ERR_INVALID;
-    if ((reinterpret_cast<uintptr_t>(ring->data) & 15) != 0) return MR_ERR_INVALID;
-    const int esz = ring->dtype == MR_F32 ? 4 : 2;
-    if (ring->dtype != MR_F32 && ring->dtype != MR_BF16 && ring->dtype != MR_F16) return MR_ERR_INVALID;
-    if ((ring->col_pitch * esz) % 16 || (ring->slot_stride * esz) % 16) return MR_ERR_INVALID;
     return MR_OK;
 }
 
