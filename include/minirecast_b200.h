@@ -293,6 +293,22 @@ int mr_mc_emit(const float* vol, int32_t nx, int32_t ny, int32_t nz, float iso,
                const double* origin, double spacing, const int64_t* block_offsets_dev,
                int64_t n_tri, int64_t* tri_edges_dev, float* tri_pos_dev, void* stream);
 
+/* The same surface as an indexed mesh: vertices shared between cells, one per crossed grid
+ * edge in the order of the edge ids above (positions as tri_pos), faces in cell order as
+ * vertex numbers.
+ * ws: device workspace of mr_mesh_workspace_bytes() bytes (16-byte aligned), written by
+ * mr_mesh_plan and read by mr_mesh_emit (the volume unchanged between the two).
+ * mr_mesh_plan: totals_host (host, 3 values) = {triangles, vertices, listed words (for
+ * mr_mesh_emit)}; the call waits for the stream. Fewer than 2^32 vertices
+ * (MR_ERR_UNSUPPORTED beyond).
+ * mr_mesh_emit: points[3 * vertices], faces[3 * triangles] (device) of those totals. */
+int64_t mr_mesh_workspace_bytes(int32_t nx, int32_t ny, int32_t nz);
+int mr_mesh_plan(const float* vol, int32_t nx, int32_t ny, int32_t nz, float iso, void* ws_dev,
+                 int64_t* totals_host, void* stream);
+int mr_mesh_emit(const float* vol, int32_t nx, int32_t ny, int32_t nz, float iso,
+                 const double* origin, double spacing, void* ws_dev, const int64_t* totals_host,
+                 float* points_dev, int64_t* faces_dev, void* stream);
+
 /* ---- raw correction alone (the scan loaders' output stack) ------------------------
  * Replaces the per-projection correction of flexray.py:111-116 + 174-184 (`corrected`,
  * mode MR_CORRECT_FLEXRAY: float32 bin mean, (mean - dark) * scale, scale = the gain

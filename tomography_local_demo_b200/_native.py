@@ -86,6 +86,9 @@ SIGNATURES = {
     "mr_mc_count": (ctypes.c_int, [_P, _I32, _I32, _I32, ctypes.c_float, _P, _P]),
     "mr_mc_emit": (ctypes.c_int, [_P, _I32, _I32, _I32, ctypes.c_float, _P, ctypes.c_double, _P, _I64, _P, _P,
                                   _P]),
+    "mr_mesh_workspace_bytes": (_I64, [_I32, _I32, _I32]),
+    "mr_mesh_plan": (ctypes.c_int, [_P, _I32, _I32, _I32, ctypes.c_float, _P, _P, _P]),
+    "mr_mesh_emit": (ctypes.c_int, [_P, _I32, _I32, _I32, ctypes.c_float, _P, ctypes.c_double, _P, _P, _P, _P, _P]),
     "mr_volume_workspace_bytes": (_I64, []),
     "mr_volume_stats": (ctypes.c_int, [_P, _I64, _P, _P, _P]),
     "mr_volume_select": (ctypes.c_int, [_P, _I64, _P, _I32, ctypes.c_uint32, ctypes.c_uint32, _P, _P, _P]),

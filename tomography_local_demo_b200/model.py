@@ -11,7 +11,8 @@ FP64-clipped values); the percentile interpolation between two order statistics 
 Otsu sums over the bins are host FP64 arithmetic on a few numbers, in numpy's order.
 
 extract_surface / marching_cubes replace the VTK (or scikit-image) contour of
-model.py:40-75 with two CUDA passes over the volume's cells (mr_mc_count, mr_mc_emit); the
+model.py:40-75 with a CUDA pass over the volume and passes over its crossed edges
+(mr_mesh_plan, mr_mesh_emit); the
 reference's connectivity filter is a device label propagation, its smoothing a Taubin
 lambda|mu pass; write_stl / save_mesh write the same binary STL as the reference.
 """
@@ -140,8 +141,8 @@ def marching_cubes(vol, iso, origin=(0.0, 0.0, 0.0), spacing=1.0):
     spacing * (i, j, k)) on the device: (points f32 tensor [V, 3], faces int64 tensor [F, 3]),
     vertices shared between cells (one per crossed grid edge, in grid-edge order), faces in
     cell order, normals (right-hand rule) pointing from values above iso to values below.
-    Two kernel passes (mr_mc_count, mr_mc_emit) with a scan of the per-block triangle
-    counts between them; vertices are merged by the grid edge they lie on."""
+    One read of the volume into inside bits, from which vertices and triangles are counted and
+    numbered (mr_mesh_plan), then both are written once (mr_mesh_emit)."""
     lib = N.load()
     t = vol if isinstance(vol, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(vol))
     if t.dtype != torch.float32 or t.dim() != 3:
@@ -155,23 +156,18 @@ def marching_cubes(vol, iso, origin=(0.0, 0.0, 0.0), spacing=1.0):
         if min(nx, ny, nz) < 2:
             return (torch.zeros((0, 3), dtype=torch.float32, device=dev),
                     torch.zeros((0, 3), dtype=torch.int64, device=dev))
-        nb = int(lib.mr_mc_blocks(nx, ny, nz))
-        counts = torch.empty(nb, dtype=torch.int32, device=dev)
-        N.check(lib.mr_mc_count(v(t.data_ptr()), nx, ny, nz, float(iso), v(counts.data_ptr()),
-                                v(stream.cuda_stream)), "mr_mc_count")
-        c64 = counts.to(torch.int64)
-        offsets = torch.cumsum(c64, 0) - c64
-        total = int(c64.sum())
-        edges = torch.empty(3 * total, dtype=torch.int64, device=dev)
-        pos = torch.empty((3 * total, 3), dtype=torch.float32, device=dev)
+        ws = torch.empty(int(lib.mr_mesh_workspace_bytes(nx, ny, nz)), dtype=torch.uint8, device=dev)
+        totals = (ctypes.c_int64 * 3)()
+        N.check(lib.mr_mesh_plan(v(t.data_ptr()), nx, ny, nz, float(iso), v(ws.data_ptr()), totals,
+                                 v(stream.cuda_stream)), "mr_mesh_plan")
+        n_tri, n_vert = int(totals[0]), int(totals[1])
+        points = torch.empty((n_vert, 3), dtype=torch.float32, device=dev)
+        faces = torch.empty((n_tri, 3), dtype=torch.int64, device=dev)
         org = (ctypes.c_double * 3)(*[float(x) for x in origin])
-        N.check(lib.mr_mc_emit(v(t.data_ptr()), nx, ny, nz, float(iso), org, float(spacing), v(offsets.data_ptr()),
-                               total, v(edges.data_ptr()) if total else None, v(pos.data_ptr()) if total else None,
-                               v(stream.cuda_stream)), "mr_mc_emit")
-        uniq, inv = torch.unique(edges, return_inverse=True)
-        points = torch.empty((len(uniq), 3), dtype=torch.float32, device=dev)
-        points[inv] = pos                       # every copy of a vertex holds the same value
-        return points, inv.view(-1, 3)
+        N.check(lib.mr_mesh_emit(v(t.data_ptr()), nx, ny, nz, float(iso), org, float(spacing), v(ws.data_ptr()),
+                                 totals, v(points.data_ptr()) if n_vert else None,
+                                 v(faces.data_ptr()) if n_tri else None, v(stream.cuda_stream)), "mr_mesh_emit")
+        return points, faces
 
 
 def _components(faces, n_points):
