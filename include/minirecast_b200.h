@@ -376,7 +376,7 @@ int mr_slice_entropy(const float* imgs, int32_t n_imgs, int64_t stride, int32_t 
  * n f32 voxels (device, 4-byte aligned, any layout): the host computes the percentile
  * interpolation and the Otsu sums over the bins in FP64 from what these return.
  * ws: device workspace of mr_volume_workspace_bytes() bytes (8-byte aligned), shared by
- * the three calls of one threshold; calls on one workspace must not overlap. */
+ * the calls of one threshold; calls on one workspace must not overlap. */
 int64_t mr_volume_workspace_bytes(void);
 
 /* Counts of the voxels != 0 and of the NaN voxels, and the order keys of the smallest
@@ -390,6 +390,18 @@ int mr_volume_stats(const float* vol, int64_t n, void* ws, uint64_t* stats_host,
  * (a radix select over the bits in which kmin and kmax, from mr_volume_stats, differ). */
 int mr_volume_select(const float* vol, int64_t n, const int64_t* ranks_host, int32_t n_ranks,
                      uint32_t kmin, uint32_t kmax, void* ws, float* values_dev, void* stream);
+
+/* The same for ranks near quantiles q_lo <= q_hi of the non-zero voxels, with one read of the
+ * volume: mr_volume_tails brackets both quantiles by a sample and collects the voxels at and
+ * beyond the brackets into ws (16-byte aligned here); stats_host (host) = {nonzero, nan, voxels
+ * of the lower tail, voxels of the upper tail}; the call waits for the stream.
+ * mr_volume_tail_select: as mr_volume_select, from the stats and the tails in ws;
+ * MR_ERR_UNSUPPORTED when a rank lies in neither tail or its tail is too large to be kept
+ * (many equal voxels): use mr_volume_stats and mr_volume_select then. */
+int mr_volume_tails(const float* vol, int64_t n, double q_lo, double q_hi, void* ws,
+                    uint64_t* stats_host, void* stream);
+int mr_volume_tail_select(const int64_t* ranks_host, int32_t n_ranks, const uint64_t* stats_host,
+                          void* ws, float* values_dev, void* stream);
 
 /* hist_dev[b] (device, bins uint64, overwritten) = the number of non-zero, non-NaN voxels
  * whose FP64 value clipped to [lo, hi] falls in bin b of numpy.histogram(..., bins,

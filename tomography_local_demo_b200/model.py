@@ -5,9 +5,10 @@ otsu_threshold(vol, bins=512) returns the reference's threshold bit for bit:
   v = vol[vol != 0]; lo, hi = np.percentile(v, [0.1, 99.95])
   hist = np.histogram(np.clip(v, lo, hi), bins, range=(lo, hi))
   argmax over the bins of w0 * w1 * (m0 - m1)^2 (Otsu's between-class variance)
-The voxel passes run as CUDA kernels (mr_volume_stats / _select / _histogram: counts and
-key range, exact order statistics by radix select, numpy's uniform-bin histogram of the
-FP64-clipped values); the percentile interpolation between two order statistics and the
+The voxel passes run as CUDA kernels (mr_volume_tails / _tail_select: counts and exact order
+statistics among the voxels beyond sampled brackets of the two percentiles, mr_volume_stats /
+_select where those do not hold them; mr_volume_histogram: numpy's uniform-bin histogram of
+the FP64-clipped values); the percentile interpolation between two order statistics and the
 Otsu sums over the bins are host FP64 arithmetic on a few numbers, in numpy's order.
 
 extract_surface / marching_cubes replace the VTK (or scikit-image) contour of
@@ -99,19 +100,25 @@ def otsu_threshold(vol, bins=512):
     with torch.cuda.device(dev):
         stream = torch.cuda.current_stream(dev)
         ws = torch.empty(int(lib.mr_volume_workspace_bytes()), dtype=torch.uint8, device=dev)
-        stats = (ctypes.c_uint64 * 3)()
-        N.check(lib.mr_volume_stats(v(t.data_ptr()) if n else None, n, v(ws.data_ptr()), stats,
-                                    v(stream.cuda_stream)), "mr_volume_stats")
-        nonzero, nan, keys = int(stats[0]), int(stats[1]), int(stats[2])
-        if nan:
+        stats = (ctypes.c_uint64 * 4)()
+        N.check(lib.mr_volume_tails(v(t.data_ptr()) if n else None, n, PERCENTILES[0] / 100, PERCENTILES[1] / 100,
+                                    v(ws.data_ptr()), stats, v(stream.cuda_stream)), "mr_volume_tails")
+        nonzero = int(stats[0])
+        if stats[1]:
             raise ValueError("supplied range of [nan, nan] is not finite")
-        kmin, kmax = keys & 0xFFFFFFFF, keys >> 32
         vals_dev = torch.empty(4, dtype=torch.float32, device=dev)
 
         def order_stat(ranks):
             r = (ctypes.c_int64 * len(ranks))(*[int(x) for x in ranks])
-            N.check(lib.mr_volume_select(v(t.data_ptr()), n, r, len(ranks), kmin, kmax, v(ws.data_ptr()),
-                                         v(vals_dev.data_ptr()), v(stream.cuda_stream)), "mr_volume_select")
+            rc = lib.mr_volume_tail_select(r, len(ranks), stats, v(ws.data_ptr()), v(vals_dev.data_ptr()),
+                                           v(stream.cuda_stream))
+            if rc == N.MR_ERR_UNSUPPORTED:          # not in the tails, or too many equal voxels to keep them
+                full = (ctypes.c_uint64 * 3)()
+                N.check(lib.mr_volume_stats(v(t.data_ptr()), n, v(ws.data_ptr()), full, v(stream.cuda_stream)),
+                        "mr_volume_stats")
+                rc = lib.mr_volume_select(v(t.data_ptr()), n, r, len(ranks), full[2] & 0xFFFFFFFF, full[2] >> 32,
+                                          v(ws.data_ptr()), v(vals_dev.data_ptr()), v(stream.cuda_stream))
+            N.check(rc, "mr_volume_select")
             return vals_dev[:len(ranks)].cpu().numpy()
 
         lo, hi = percentile_linear(nonzero, PERCENTILES, order_stat)
