@@ -76,42 +76,49 @@ class BackprojectOp:
         """B q with the coordinate arithmetic of the backward kernels (mr_backproject_matched)."""
         out = torch.zeros(self.n_out, dtype=torch.float32, device=self.device)
         grids = self.grids_at(shift, tilt)
-        g_dev, t_dev = self._tiles(grids)
+        recs, tiles, n_tiles = self._tiles(grids)
         st = torch.cuda.current_stream(self.device)
         v = ctypes_void
-        N.check(N.load().mr_backproject_matched(self._ring(q), v(self.views.data_ptr()), v(g_dev.data_ptr()),
-                                                v(t_dev.data_ptr()), t_dev.numel() // N.TILE_DTYPE.itemsize,
+        N.check(N.load().mr_backproject_matched(self._ring(q), v(self.views.data_ptr()), v(recs.data_ptr()),
+                                                tiles, n_tiles,
                                                 v(out.data_ptr()), v(st.cuda_stream)), "mr_backproject_matched")
         return out
 
     def _tiles(self, grids):
-        return _struct_tensor(grids, self.device), _struct_tensor(N.plan_tiles(grids), self.device)
+        """(device records: grids, then their tiles; pointer to the tiles; how many). One upload
+        through page-locked staging, so the call does not wait for what the stream still has to
+        do; while a graph is captured, the copy that a capture refuses (its staging would not
+        hold the records at a replay)."""
+        tiles = N.plan_tiles(grids)
+        recs = np.concatenate([grids.view(np.uint8), tiles.view(np.uint8)])
+        dev = _struct_tensor(recs, self.device, asynchronous=not torch.cuda.is_current_stream_capturing())
+        return dev, ctypes_void(dev.data_ptr() + grids.nbytes), len(tiles)
 
     def adjoint(self, gout, shift=0.0, tilt=0.0, shape=None):
         """B^T gout as an f32 tensor of `shape` ([views, rows, pitch])."""
         shape = shape or (self.n_views, self.rows, self.cols)
         gq = torch.zeros(shape, dtype=torch.float32, device=self.device)
         grids = self.grids_at(shift, tilt)
-        g_dev, t_dev = self._tiles(grids)
+        recs, tiles, n_tiles = self._tiles(grids)
         st = torch.cuda.current_stream(self.device)
         gout = gout.to(torch.float32).contiguous()
         ring = _ring_struct(gq, N.MR_F32, self.kind, self.rows, self.cols)
         v = ctypes_void
-        N.check(N.load().mr_project_adjoint(ring, v(self.views.data_ptr()), v(g_dev.data_ptr()),
-                                            v(t_dev.data_ptr()), t_dev.numel() // N.TILE_DTYPE.itemsize,
+        N.check(N.load().mr_project_adjoint(ring, v(self.views.data_ptr()), v(recs.data_ptr()),
+                                            tiles, n_tiles,
                                             v(gout.data_ptr()), v(st.cuda_stream)), "mr_project_adjoint")
         return gq
 
     def grad_geometry(self, q, gout, shift=0.0, tilt=0.0):
         """(d<gout, B q>/dshift, d<gout, B q>/dtilt) summed over the grids."""
         grids = self.grids_at(shift, tilt)
-        g_dev, t_dev = self._tiles(grids)
+        recs, tiles, n_tiles = self._tiles(grids)
         d = torch.zeros(2 * len(grids), dtype=torch.float64, device=self.device)
         st = torch.cuda.current_stream(self.device)
         gout = gout.to(torch.float32).contiguous()
         v = ctypes_void
-        N.check(N.load().mr_bp_grad_geom(self._ring(q), v(self.views.data_ptr()), v(g_dev.data_ptr()),
-                                         v(t_dev.data_ptr()), t_dev.numel() // N.TILE_DTYPE.itemsize,
+        N.check(N.load().mr_bp_grad_geom(self._ring(q), v(self.views.data_ptr()), v(recs.data_ptr()),
+                                         tiles, n_tiles,
                                          v(gout.data_ptr()), v(d.data_ptr()), v(st.cuda_stream)),
                 "mr_bp_grad_geom")
         d = d.view(-1, 2).sum(0)

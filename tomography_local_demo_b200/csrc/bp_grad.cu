@@ -31,18 +31,54 @@ namespace mr {
 
 constexpr int GR_THREADS = 256;
 constexpr int GR_PPT = 4;
+constexpr int GR_DI = GR_THREADS / 32;         // row step between a thread's samples
 constexpr int GR_VCH = 128;
+constexpr int GR_TILE = 32;                    // tile edge (samples), as planned by mr_plan_tiles
 
 enum : int { GRAD_ADJOINT = 0, GRAD_GEOM = 1, GRAD_FORWARD = 2 };
 
+// Where the footprint of a whole 32 x 32 tile lies in a view: wholly on the detector with a
+// margin of half a pixel (no tap of any lane needs a check), wholly off it (nothing to add),
+// or neither. The tile's four corners bound it: it is planar, and in front of the source.
+enum : int { FOOT_EDGE = 0, FOOT_INSIDE = 1, FOOT_OFF = 2 };
+
+template <int KIND>
+__device__ __forceinline__ int tile_footprint(const float* pu, const float* pv, const float* pw, const mr_grid& g,
+                                              const mr_tile& t, int R, int C) {
+    float cmin = 3e38f, cmax = -3e38f, rmin = 3e38f, rmax = -3e38f;
+    bool front = true;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float i = (float)(t.i0 + ((c & 1) ? GR_TILE - 1 : 0)), j = (float)(t.j0 + ((c & 2) ? GR_TILE - 1 : 0));
+        float p[3];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) p[e] = g.origin[e] + i * g.step_i[e] + j * g.step_j[e] + t.k * g.step_k[e];
+        float col = fmaf(pu[0], p[0], fmaf(pu[1], p[1], fmaf(pu[2], p[2], pu[3])));
+        float row = fmaf(pv[0], p[0], fmaf(pv[1], p[1], fmaf(pv[2], p[2], pv[3])));
+        if (KIND == MR_CONE) {
+            const float w = fmaf(pw[0], p[0], fmaf(pw[1], p[1], fmaf(pw[2], p[2], pw[3])));
+            front = front && w > 1e-3f;
+            col /= w;
+            row /= w;
+        }
+        cmin = fminf(cmin, col); cmax = fmaxf(cmax, col);
+        rmin = fminf(rmin, row); rmax = fmaxf(rmax, row);
+        front = front && col == col && row == row;
+    }
+    if (!front) return FOOT_EDGE;
+    if (cmax < -2.f || rmax < -2.f || cmin > (float)C + 1.f || rmin > (float)R + 1.f) return FOOT_OFF;
+    return cmin > 0.5f && rmin > 0.5f && cmax < (float)C - 1.5f && rmax < (float)R - 1.5f ? FOOT_INSIDE : FOOT_EDGE;
+}
+
 template <int KIND, int MODE, typename T>
-__global__ void __launch_bounds__(GR_THREADS)
+__global__ void __launch_bounds__(GR_THREADS, 3)
 bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int C, int pitch,
                long long slot_stride, int n_slots, const mr_view* __restrict__ views,
                const mr_grid* __restrict__ grids,
                const mr_tile* __restrict__ tiles, const float* __restrict__ gout, double* __restrict__ dgeom) {
     __shared__ float4 s_u[GR_VCH], s_v[GR_VCH], s_w[GR_VCH];
     __shared__ float s_q[GR_VCH], s_uv[GR_VCH];
+    __shared__ int s_foot[GR_VCH];
     __shared__ mr_grid s_g;
     __shared__ double s_red[2][GR_THREADS / 32];
     __shared__ float4 s_part[GR_THREADS];
@@ -57,8 +93,11 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
     const mr_grid& g = s_g;
     const bool pts = (g.flags & MR_GRID_POINTS) != 0;
     const int warp = tid >> 5, lane = tid & 31;
-    const int tx = ((warp & 3) << 3) | (lane & 7);
-    const int ty = ((warp >> 2) << 4) | (lane >> 3);
+    // a warp takes rows of 32 samples along j, eight rows apart: on a slice j is horizontal, so
+    // a row's taps lie on one or two detector rows and a warp-wide gather or reduction touches
+    // few lines (8 x 4 patches: forward 505, adjoint 830, geometry 497 us where this takes 459,
+    // 705 and 459 with the calls' records; one 512^2 slice, 600 views of 486 x 384)
+    const int tx = lane, ty = warp;
 
     float px[GR_PPT], py[GR_PPT], pz[GR_PPT], gp[GR_PPT], acc[GR_PPT];
     long long oidx[GR_PPT];
@@ -74,7 +113,7 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
             ok = j < g.n_j;
             o = g.out_offset + (long long)j * g.out_stride_j;
         } else {
-            i = t.i0 + ty + 4 * p;
+            i = t.i0 + ty + GR_DI * p;
             j = t.j0 + tx;
             ok = i < g.n_i && j < g.n_j;
             o = g.out_offset + (long long)i * g.out_stride_i + (long long)j * g.out_stride_j +
@@ -106,6 +145,11 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
             pz[p] = g.origin[2] + i * g.step_i[2] + j * g.step_j[2] + t.k * g.step_k[2];
         }
     }
+    // a warp none of whose samples counts has nothing to do in the view loop
+    bool own = false;
+#pragma unroll
+    for (int p = 0; p < GR_PPT; ++p) own |= MODE == GRAD_FORWARD ? live[p] : gp[p] != 0.f;
+    const bool busy = __any_sync(0xffffffffu, own);
     const float shift = g.cor_shift;
     const float cc = 0.5f * (float)(C - 1), cr = 0.5f * (float)(R - 1);
     float ds = 0.f, dt = 0.f;
@@ -129,12 +173,74 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
             s_w[tid] = make_float4(V.pw[0], V.pw[1], V.pw[2], V.pw[3]);
             s_q[tid] = V.qscale;
             s_uv[tid] = V.uv;
+            s_foot[tid] = pts ? FOOT_EDGE : tile_footprint<KIND>(pu, pv, V.pw, g, t, R, C);
         }
         __syncthreads();
         for (int vv = 0; vv < nch; ++vv) {
+            const int foot = s_foot[vv];
+            if (foot == FOOT_OFF || !busy) continue;
             const float4 cu = s_u[vv], cv = s_v[vv], cw = s_w[vv];
             const float qs = s_q[vv], uv = s_uv[vv];
             const long long slot = (long long)(first + v0 + vv) * slot_stride;
+            if (foot == FOOT_INSIDE) {
+                // The arithmetic of the general path below without its checks, the taps of all
+                // four samples in flight together: with a branch between the samples each one
+                // waited for its own loads.
+                float col[GR_PPT], row[GR_PPT], w[GR_PPT], fr[GR_PPT], fc[GR_PPT];
+                float q00[GR_PPT], q01[GR_PPT], q10[GR_PPT], q11[GR_PPT];
+                int off[GR_PPT];
+#pragma unroll
+                for (int p = 0; p < GR_PPT; ++p) {
+                    col[p] = fmaf(cu.x, px[p], fmaf(cu.y, py[p], fmaf(cu.z, pz[p], cu.w)));
+                    row[p] = fmaf(cv.x, px[p], fmaf(cv.y, py[p], fmaf(cv.z, pz[p], cv.w)));
+                    w[p] = qs;
+                    if (KIND == MR_CONE) {
+                        const float r = rcp_approx(fmaf(cw.x, px[p], fmaf(cw.y, py[p], fmaf(cw.z, pz[p], cw.w))));
+                        col[p] *= r;
+                        row[p] *= r;
+                        w[p] *= r * r;
+                    }
+                    const float r0f = floorf(row[p]), c0f = floorf(col[p]);
+                    fr[p] = row[p] - r0f;
+                    fc[p] = col[p] - c0f;
+                    off[p] = (int)r0f * pitch + (int)c0f;
+                }
+                if (MODE != GRAD_ADJOINT) {
+                    const T* __restrict__ q = ring + slot;
+#pragma unroll
+                    for (int p = 0; p < GR_PPT; ++p) {
+                        const T* a = q + off[p];
+                        q00[p] = ld_elem(a);
+                        q01[p] = ld_elem(a + 1);
+                        q10[p] = ld_elem(a + pitch);
+                        q11[p] = ld_elem(a + pitch + 1);
+                    }
+                }
+#pragma unroll
+                for (int p = 0; p < GR_PPT; ++p) {
+                    if (MODE == GRAD_FORWARD) {             // samples that are not live are not written
+                        const float a = fmaf(fc[p], q01[p] - q00[p], q00[p]);
+                        const float b = fmaf(fc[p], q11[p] - q10[p], q10[p]);
+                        acc[p] = fmaf(w[p], fmaf(fr[p], b - a, a), acc[p]);
+                    } else if (MODE == GRAD_ADJOINT) {
+                        if (gp[p] != 0.f) {
+                            float* o = gring + slot + off[p];
+                            const float a = w[p] * gp[p];
+                            atomicAdd(o, a * (1.f - fr[p]) * (1.f - fc[p]));
+                            atomicAdd(o + 1, a * (1.f - fr[p]) * fc[p]);
+                            atomicAdd(o + pitch, a * fr[p] * (1.f - fc[p]));
+                            atomicAdd(o + pitch + 1, a * fr[p] * fc[p]);
+                        }
+                    } else if (gp[p] != 0.f) {
+                        const float dcol = fmaf(fr[p], q11[p] - q10[p], (1.f - fr[p]) * (q01[p] - q00[p]));
+                        const float drow = fmaf(fc[p], q11[p] - q01[p], (1.f - fc[p]) * (q10[p] - q00[p]));
+                        const float a = w[p] * gp[p];
+                        ds = fmaf(a, fmaf(drow, uv, dcol), ds);
+                        dt = fmaf(a, dcol * (row[p] - shift * uv - cr) - drow * (col[p] - shift - cc), dt);
+                    }
+                }
+                continue;
+            }
 #pragma unroll
             for (int p = 0; p < GR_PPT; ++p) {
                 if (MODE == GRAD_FORWARD ? !live[p] : gp[p] == 0.f) continue;
@@ -199,7 +305,7 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
 #pragma unroll
         for (int p = 0; p < GR_PPT; ++p) {
             const bool ok = pts ? (t.j0 + tid + GR_THREADS * p < g.n_j)
-                                : (t.i0 + ty + 4 * p < g.n_i && t.j0 + tx < g.n_j);
+                                : (t.i0 + ty + GR_DI * p < g.n_i && t.j0 + tx < g.n_j);
             if (ok) {
                 const float val = live[p] ? acc[p] * g.scale : 0.f;
                 gring[oidx[p]] = g.accumulate ? gring[oidx[p]] + val : val;
@@ -227,12 +333,14 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
 template <int KIND, int MODE, typename T>
 static int launch_grad(const mr_ring* ring, float* gring, const mr_view* views, const mr_grid* grids,
                        const mr_tile* tiles, int64_t n_tiles, const float* gout, double* dgeom, cudaStream_t st) {
-    // CTAs per tile: enough for about four waves of CTAs on the GPU, at most 8 (portable cluster)
+    // CTAs per tile: enough for about five waves of three CTAs an SM, at most 8 (portable
+    // cluster). Tiles differ in how many of their samples count, so short CTAs even out (256
+    // tiles: 8 CTAs each 551, 4 each 698 us for the geometry gradient)
     int dev = 0, sms = 148;
     MR_CUDA_TRY(cudaGetDevice(&dev));
     MR_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int cl = 1;
-    while (cl < 8 && n_tiles * cl < 4LL * sms) cl *= 2;
+    while (cl < 8 && n_tiles * cl < 16LL * sms) cl *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GR_THREADS);
     cfg.stream = st;
