@@ -68,24 +68,32 @@ __global__ void gauss_axis_kernel(const float* __restrict__ in, float* __restric
 // the padded length (the spectrum is cut at Nyquist), so a direct loop costs ~n/2 taps per
 // output. A block takes L lines (rows along axis 2, columns along axis 0) and TO outputs of
 // each: it stages the stretch of the edge-padded, periodically extended line those outputs
-// read into shared memory once, then every thread computes 8 consecutive outputs of one
-// line, 8 taps at a time: 15 staged values in registers serve the 64 products of a block of
-// taps. The taps are padded in front with zeros to a multiple of 8 (m from K - 8 nb + 1);
-// those add 0 * x to a zero sum, exactly, so each output is the same FMA chain over
-// m = -K .. K as in gauss_axis_kernel and the results are identical.
+// read into shared memory once, then every thread computes 16 consecutive outputs of two
+// neighbouring lines, 8 taps at a time. Both lines share every instruction (packed f32x2
+// multiply-adds), and the 23 staged positions that a block of 8 taps reaches stay in
+// registers from one block to the next, 8 new ones a block: 128 packed multiply-adds on 12
+// shared-memory loads. The taps are padded in front with zeros to a multiple of 8 (m from
+// K - 8 nb + 1); those add 0 * x to a zero sum, exactly, so each output is the same FMA chain
+// over m = -K .. K as in gauss_axis_kernel and the results are identical.
+// Bound by the FMA pipe (64 views of 486 x 384, sigma 1, 390 and 492 taps an output: rows 328 ->
+// 222 us, columns 465 -> 278 us, 60 % of its rate, of them about 60 and 90 us staging and
+// stores). Before, a thread computed 8 outputs of one line and loaded its 15 positions anew for
+// every block of taps; without the unrolling by 3 the window's moves cost 10 %.
 constexpr int GS_THREADS = 256;
-constexpr int GS_RUN = 8;                       // consecutive outputs per thread = taps per block
+constexpr int GS_TAPS = 8;                      // taps per block
+constexpr int GS_RUN = 16;                      // consecutive outputs per thread
 
 template <int L, int LP>
-__global__ void __launch_bounds__(GS_THREADS)
+__global__ void __launch_bounds__(GS_THREADS, 2)
 gauss_lines_kernel(const float* __restrict__ in, float* __restrict__ out, int R, int A, int C, int axis,
                    int pad, const float* __restrict__ g, int K, int TO) {
-    extern __shared__ float gsm[];
-    const int nb = (2 * K + 1 + GS_RUN - 1) / GS_RUN;           // blocks of 8 taps
-    const int m0 = K - GS_RUN * nb + 1;                        // first (zero-padded) tap
-    const int T = TO + GS_RUN * nb;             // staged positions per line
-    float* taps = gsm;                          // [8 nb]: tap m0 + i
-    float* ext = gsm + GS_RUN * nb;             // [T][LP]
+    static_assert(L % 2 == 0 && LP % 2 == 0, "lines in pairs");
+    extern __shared__ __align__(16) float gsm[];
+    const int nb = (2 * K + GS_TAPS) / GS_TAPS;                 // blocks of 8 taps
+    const int m0 = K - GS_TAPS * nb + 1;                       // first (zero-padded) tap
+    const int T = TO + GS_TAPS * nb;            // staged positions per line
+    float2* taps = reinterpret_cast<float2*>(gsm);              // [8 nb]: tap m0 + i, twice
+    float* ext = gsm + 2 * GS_TAPS * nb;        // [T][LP]
     const long long srow = (long long)A * C;
     const int n = axis == 0 ? R : C;
     const int Np = n + 2 * pad;
@@ -98,64 +106,105 @@ gauss_lines_kernel(const float* __restrict__ in, float* __restrict__ out, int R,
         const long long r = line / A, a = line - r * A;
         return r * srow + a * C;
     };
-    for (int i = threadIdx.x; i < GS_RUN * nb; i += GS_THREADS) {
+    for (int i = threadIdx.x; i < GS_TAPS * nb; i += blockDim.x) {
         const int m = m0 + i;
-        taps[i] = m < -K ? 0.f : __ldg(g + (m < 0 ? -m : m));
+        const float v = m < -K ? 0.f : __ldg(g + (m < 0 ? -m : m));
+        taps[i] = make_float2(v, v);
     }
-    // staged position t holds padded position i0 + pad - K + t; output o at tap m reads t = o + K - m
+    // staged position t holds padded position i0 + pad - K + t; output o at tap m reads t = o + K - m.
+    // The line position behind it (circular, edge padding) is the same for every line: a table,
+    // then asynchronous copies that need only an address each.
     const int nl = (int)min((long long)L, n_lines - line0);
-    for (int e = threadIdx.x; e < L * T; e += GS_THREADS) {
-        int l, t;
-        if (axis == 0) { l = e % L; t = e / L; }                        // neighbouring columns
-        else { l = e / T; t = e - (e / T) * T; }                        // along one row
-        float v = 0.f;
-        if (l < nl) {
-            int u = i0 + pad - K + t;                                   // padded position
-            u %= Np;
-            if (u < 0) u += Np;                                         // circular
-            int src = u - pad;                                          // edge padding
-            src = src < 0 ? 0 : (src >= n ? n - 1 : src);
-            v = __ldg(in + line_base(line0 + l) + src * step);
-        }
-        ext[t * LP + l] = v;
+    int* from = reinterpret_cast<int*>(ext + T * LP);           // [T]
+    for (int t = threadIdx.x; t < T; t += blockDim.x) {
+        int u = i0 + pad - K + t;                                       // padded position
+        u %= Np;
+        if (u < 0) u += Np;                                             // circular
+        from[t] = min(max(u - pad, 0), n - 1);                          // edge padding
     }
     __syncthreads();
+    const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(ext));
+    auto copy = [&](int t, int l, const float* src) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to + (t * LP + l) * 4), "l"(src) : "memory");
+    };
+    if (axis == 0) {                                                    // lanes along neighbouring columns
+        const int l = threadIdx.x % L;
+        if (l < nl) {
+            const float* line = in + line0 + l;
+#pragma unroll 4
+            for (int t = threadIdx.x / L; t < T; t += blockDim.x / L) copy(t, l, line + from[t] * step);
+        }
+    } else {                                                            // lanes along one row
+        const int lane = threadIdx.x & 31;
+        for (int l = threadIdx.x >> 5; l < nl; l += blockDim.x >> 5) {
+            const float* line = in + line_base(line0 + l);
+#pragma unroll 4
+            for (int t = lane; t < T; t += 32) copy(t, l, line + from[t]);
+        }
+    }
+    if (nl & 1)                                                         // a pair's missing line
+        for (int t = threadIdx.x; t < T; t += blockDim.x) ext[t * LP + nl] = 0.f;
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
     const int groups = (TO + GS_RUN - 1) / GS_RUN;
-    for (int task = threadIdx.x; task < L * groups; task += GS_THREADS) {
-        const int l = task % L, q = task / L;
+    for (int task = threadIdx.x; task < L / 2 * groups; task += blockDim.x) {
+        const int l = 2 * (task % (L / 2)), q = task / (L / 2);         // lines l, l + 1
         const int o0 = q * GS_RUN;                                      // first output (block-local)
         if (l >= nl || i0 + o0 >= n) continue;
-        float acc[GS_RUN];
+        float2 acc[GS_RUN];
 #pragma unroll
-        for (int j = 0; j < GS_RUN; ++j) acc[j] = 0.f;
+        for (int j = 0; j < GS_RUN; ++j) acc[j] = make_float2(0.f, 0.f);
+        // taps m0 + 8 b + u (u < 8) of output o0 + j read position first + 8 (nb - 1 - b) + 7 + j - u;
+        // w holds the block's positions .. + 0 .. 22
+        const float2* p = reinterpret_cast<const float2*>(ext + (o0 + K - m0 - (GS_TAPS - 1)) * LP + l);
+        float2 w[GS_RUN + GS_TAPS - 1];
+#pragma unroll
+        for (int k = GS_TAPS; k < GS_RUN + GS_TAPS - 1; ++k) w[k] = p[k * (LP / 2)];
+#pragma unroll 3                                // the window's three parts change names, not registers
         for (int b = 0; b < nb; ++b) {
-            // taps m = mb + u (u < 8) of outputs o0 + j read t = o0 + j + K - mb - u
-            const int base = o0 + K - (m0 + GS_RUN * b) - (GS_RUN - 1);
-            float w[2 * GS_RUN - 1];
 #pragma unroll
-            for (int k = 0; k < 2 * GS_RUN - 1; ++k) w[k] = ext[(base + k) * LP + l];
+            for (int k = 0; k < GS_TAPS; ++k) w[k] = p[k * (LP / 2)];
 #pragma unroll
-            for (int u = 0; u < GS_RUN; ++u) {
-                const float gm = taps[GS_RUN * b + u];
+            for (int u = 0; u < GS_TAPS; ++u) {
+                const float2 gm = taps[GS_TAPS * b + u];
 #pragma unroll
-                for (int j = 0; j < GS_RUN; ++j) acc[j] = fmaf(gm, w[j - u + GS_RUN - 1], acc[j]);
+                for (int j = 0; j < GS_RUN; ++j) acc[j] = __ffma2_rn(gm, w[j - u + GS_TAPS - 1], acc[j]);
             }
+#pragma unroll
+            for (int k = GS_RUN + GS_TAPS - 2; k >= GS_TAPS; --k) w[k] = w[k - GS_TAPS];
+            p -= GS_TAPS * (LP / 2);
         }
-        const long long lb = line_base(line0 + l);
+        const long long lb0 = line_base(line0 + l), lb1 = line_base(min(line0 + l + 1, n_lines - 1));
 #pragma unroll
         for (int j = 0; j < GS_RUN; ++j) {
             const int i = i0 + o0 + j;
-            if (i < n && o0 + j < TO) out[lb + (long long)i * step] = acc[j];
+            if (i >= n || o0 + j >= TO) continue;
+            out[lb0 + (long long)i * step] = acc[j].x;
+            if (l + 1 < nl) out[lb1 + (long long)i * step] = acc[j].y;
         }
     }
 }
 
-// LP: the staged line stride (L + 1, or 18 for 16 lines: the two half-warps of a warp,
-// 8 staged positions apart, then fall on opposite halves of the banks)
 template <int LP>
 static size_t gauss_lines_smem(int K, int TO) {
-    const int nb = (2 * K + 1 + GS_RUN - 1) / GS_RUN;
-    return ((size_t)(TO + GS_RUN * nb) * LP + (size_t)GS_RUN * nb) * sizeof(float);
+    const int nb = (2 * K + GS_TAPS) / GS_TAPS;
+    return ((size_t)(TO + GS_TAPS * nb) * (LP + 1) + 2 * (size_t)GS_TAPS * nb) * sizeof(float);
+}
+
+template <int L, int LP>
+static int launch_gauss_lines(const float* in, float* out, int R, int A, int C, int axis, int pad, const float* taps,
+                              int K, int TO, cudaStream_t st) {
+    const int n = axis == 0 ? R : C;
+    const long long n_lines = axis == 0 ? (long long)A * C : (long long)R * A;
+    const size_t smem = gauss_lines_smem<LP>(K, TO);
+    MR_CUDA_TRY(cudaFuncSetAttribute(gauss_lines_kernel<L, LP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem));
+    // no more threads than tasks (rounded to warps), but four warps for the staging
+    const int tasks = L / 2 * ((TO + GS_RUN - 1) / GS_RUN);
+    const int threads = tasks < 128 ? 128 : (tasks < GS_THREADS ? (tasks + 31) / 32 * 32 : GS_THREADS);
+    const dim3 grid((unsigned)((n_lines + L - 1) / L), (unsigned)((n + TO - 1) / TO));
+    gauss_lines_kernel<L, LP><<<grid, threads, smem, st>>>(in, out, R, A, C, axis, pad, taps, K, TO);
+    return MR_OK;
 }
 
 }  // namespace mr
@@ -184,25 +233,16 @@ extern "C" int mr_gaussian_axis_f32(const float* in, float* out, int32_t rows, i
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int K = n_taps - 1;
     const int n = axis == 0 ? rows : cols;
-    const long long n_lines = axis == 0 ? (long long)k * cols : (long long)rows * k;
     constexpr size_t kSmemMax = 200 * 1024;
     // whole lines per block (16 lines: every input staged about twice, the periodic
-    // extension) where they fit, else 8 lines x 256 outputs
+    // extension) where they fit, else 8 lines x 512 outputs
     const int whole = (n + mr::GS_RUN - 1) / mr::GS_RUN * mr::GS_RUN;
     if (K <= n + 2 * pad && mr::gauss_lines_smem<18>(K, whole) <= kSmemMax) {
-        const size_t smem = mr::gauss_lines_smem<18>(K, whole);
-        MR_CUDA_TRY(cudaFuncSetAttribute(mr::gauss_lines_kernel<16, 18>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        const dim3 grid((unsigned)((n_lines + 15) / 16), 1);
-        mr::gauss_lines_kernel<16, 18><<<grid, mr::GS_THREADS, smem, st>>>(in, out, rows, k, cols, axis, pad, taps,
-                                                                            K, whole);
-    } else if (K <= n + 2 * pad && mr::gauss_lines_smem<9>(K, 256) <= kSmemMax) {
-        const size_t smem = mr::gauss_lines_smem<9>(K, 256);
-        MR_CUDA_TRY(cudaFuncSetAttribute(mr::gauss_lines_kernel<8, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
-        const dim3 grid((unsigned)((n_lines + 7) / 8), (unsigned)((n + 255) / 256));
-        mr::gauss_lines_kernel<8, 9><<<grid, mr::GS_THREADS, smem, st>>>(in, out, rows, k, cols, axis, pad, taps, K,
-                                                                          256);
+        const int rc = mr::launch_gauss_lines<16, 18>(in, out, rows, k, cols, axis, pad, taps, K, whole, st);
+        if (rc != MR_OK) return rc;
+    } else if (K <= n + 2 * pad && mr::gauss_lines_smem<10>(K, 512) <= kSmemMax) {
+        const int rc = mr::launch_gauss_lines<8, 10>(in, out, rows, k, cols, axis, pad, taps, K, 512, st);
+        if (rc != MR_OK) return rc;
     } else {
         const dim3 block(128);
         const dim3 grid((cols + 127) / 128, rows, k);
