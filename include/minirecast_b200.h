@@ -169,6 +169,13 @@ int mr_backproject_staged(const mr_ring* ring, const mr_view* views_dev,
                           const mr_grid* grids_dev, const mr_tile* tiles_dev, int64_t n_tiles,
                           float* out_dev, int32_t* status_dev, void* stream);
 
+/* The same, bit for bit, for grids whose samples lie a few detector pixels apart: footprints of
+ * a tile that are wide and flat (up to 252 columns x 16 rows or 168 x 32; 248 x 24 or 176 x 40
+ * for 16-bit rings) are staged too, where mr_backproject_staged reads global memory. */
+int mr_backproject_staged_wide(const mr_ring* ring, const mr_view* views_dev,
+                               const mr_grid* grids_dev, const mr_tile* tiles_dev, int64_t n_tiles,
+                               float* out_dev, int32_t* status_dev, void* stream);
+
 /* The same sum over one regular grid (no flags) that is deep along i, j and k: a volume,
  * in blocks of 16 x 16 x 16 voxels whose footprints are staged once per view. Views whose
  * detector column and depth do not change along j (the volume's z on the usual orbit) share

@@ -62,6 +62,7 @@ SIGNATURES = {
     "mr_plan_tiles": (ctypes.c_int, [_P, _I32, _P, _I64, ctypes.POINTER(_I64)]),
     "mr_backproject": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P]),
     "mr_backproject_staged": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P, _P]),
+    "mr_backproject_staged_wide": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P, _P]),
     "mr_backproject_volume": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _P]),
     "mr_backproject_persistent": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _I64, _P, _P, _P, _P]),
     "mr_backproject_persistent_noalloc": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _I64, _P, _P, _P]),

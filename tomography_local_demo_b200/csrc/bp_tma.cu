@@ -36,9 +36,19 @@ template <typename T> struct StageGeom;
 // across banks (88 bf16 = 44 words, 84 f32 = 84 words). MAXB boxes of 8 rows per stage:
 // FP32 stages hold 64 rows, so three CTAs fit an SM (80-row FP32 stages allowed two, and
 // the three-slice launch ran 18 % slower); taller footprints use the global-load path.
-template <> struct StageGeom<__nv_bfloat16> { static constexpr int W = 88, ALIGN = 8, STAGES = 4, MAXB = 10; };
-template <> struct StageGeom<__half> { static constexpr int W = 88, ALIGN = 8, STAGES = 4, MAXB = 10; };
-template <> struct StageGeom<float> { static constexpr int W = 84, ALIGN = 4, STAGES = 3, MAXB = 8; };
+// W2 / W3: the same stage as fewer, wider boxes, for footprints that are wide and flat - a tile
+// of an axial slice at a few pixels a sample covers 100 to 250 columns and two or three rows
+// (25 axial slices of 192^2, 600 views of 486 x 384, FP32: 1739 us with the global-load path
+// for them, 1003 us with these). A variant of the kernel, as the branch costs launches without
+// such footprints 8 % (three 512^2 slices 508 -> 549 us).
+template <> struct StageGeom<__nv_bfloat16> {
+    static constexpr int W = 88, ALIGN = 8, STAGES = 4, MAXB = 10, W2 = 176, MAXB2 = 5, W3 = 248, MAXB3 = 3;
+};
+template <> struct StageGeom<__half> : StageGeom<__nv_bfloat16> {};
+template <> struct StageGeom<float> {
+    static constexpr int W = 84, ALIGN = 4, STAGES = 3, MAXB = 8, W2 = 168, MAXB2 = 4, W3 = 252, MAXB3 = 2;
+};
+enum : int { MODE_WIDE2 = 3, MODE_WIDE3 = 4 };       // beside MODE_STAGED / MODE_GLOBAL / MODE_SKIP
 
 
 // What the consumer warps read per (tile, view): the local affine maps of the projective
@@ -48,10 +58,13 @@ template <> struct StageGeom<float> { static constexpr int W = 84, ALIGN = 4, ST
 struct __align__(16) ViewRec {
     float4 a, b, c;
 };
-// The producer's copy adds the TMA box origin and count.
+// The producer's copy adds the TMA box origin and count. Wide modes keep detector coordinates
+// (the arithmetic of the global path, bit for bit); `origin` is then the offset that the
+// magic-constant bits of (r0, x0) have.
 struct __align__(16) ViewMeta {
     ViewRec rec;
     int x0, r0, nbox, mode;
+    uint32_t origin;
 };
 
 __device__ __forceinline__ bool in_box_fp64_t(const mr_grid& g, int i, int j) {
@@ -69,7 +82,7 @@ __device__ __forceinline__ bool in_box_fp64_t(const mr_grid& g, int i, int j) {
 
 // Per-view footprint + local affine coefficients of one tile (computed by one lane of
 // the producer warp).
-template <int KIND, typename T>
+template <int KIND, bool WIDE, typename T>
 __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g, float ox, float oy,
                                               float oz, int di_max, int dj_max, int R, int C) {
     constexpr int W = StageGeom<T>::W;
@@ -119,6 +132,14 @@ __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g
             nbox = (rows + ST_BOX_H - 1) / ST_BOX_H;
             if ((int)floorf(cmax) + 3 - x0 <= W && nbox <= StageGeom<T>::MAXB) mode = MODE_STAGED;
         }
+        if (WIDE && mode == MODE_GLOBAL && cmax - cmin < 256.f && rmax - rmin < 64.f) {
+            x0 = ((int)floorf(cmin) - 1) & ~(StageGeom<T>::ALIGN - 1);
+            r0 = (int)floorf(rmin) - 1;
+            const int wide = (int)floorf(cmax) + 3 - x0;
+            nbox = ((int)floorf(rmax) + 3 - r0 + ST_BOX_H - 1) / ST_BOX_H;
+            if (wide <= StageGeom<T>::W2 && nbox <= StageGeom<T>::MAXB2) mode = MODE_WIDE2;
+            else if (wide <= StageGeom<T>::W3 && nbox <= StageGeom<T>::MAXB3) mode = MODE_WIDE3;
+        }
     }
     float3 cu = au, cv = av;
     if (mode == MODE_STAGED) {
@@ -128,7 +149,10 @@ __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g
     }
     // largest byte offset of a tap pair's left tap inside the staged boxes
     constexpr int ESZ = (int)sizeof(T);
-    const uint32_t maxoff = mode == MODE_STAGED ? (uint32_t)(nbox * W * ST_BOX_H * ESZ - (W + 1) * ESZ - ESZ) : 0u;
+    const int wcols = mode == MODE_WIDE2 ? StageGeom<T>::W2 : (mode == MODE_WIDE3 ? StageGeom<T>::W3 : W);
+    const bool boxes = mode != MODE_GLOBAL && mode != MODE_SKIP;
+    const uint32_t maxoff = boxes ? (uint32_t)(nbox * wcols * ST_BOX_H * ESZ - (wcols + 1) * ESZ - ESZ) : 0u;
+    m.origin = (uint32_t)(MAGIC_BITS + r0) * (uint32_t)(wcols * ESZ) + (uint32_t)(MAGIC_BITS + x0) * (uint32_t)ESZ;
     m.rec.a = make_float4(cu.x, cu.y, cu.z, cv.x);
     m.rec.b = make_float4(cv.y, cv.z, aw.x, aw.y);
     m.rec.c = make_float4(aw.z, V.qscale, __uint_as_float(maxoff), __int_as_float(mode));
@@ -145,9 +169,10 @@ __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g
 // (DSMEM) in rank order - deterministic, no atomics, no scratch - and writes the tile.
 // Three CTAs fit an SM (shared memory); the launch bound says so, or ptxas aims at four and
 // spills the FP32 variant to fit its registers.
-template <int KIND, typename T>
+template <int KIND, bool WIDE, typename T>
 __global__ void __launch_bounds__(ST_THREADS, 3)
-bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__ ring, int R, int C,
+bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap2,
+                 const __grid_constant__ CUtensorMap tmap3, const T* __restrict__ ring, int R, int C,
                  int pitch, long long slot_stride, int n_slots, const mr_view* __restrict__ views,
                  const mr_grid* __restrict__ grids, const mr_tile* __restrict__ tiles,
                  float* __restrict__ out, int* status, const int64_t* __restrict__ n_tiles_dev,
@@ -159,6 +184,11 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__
     constexpr int BOX_BYTES = W * ST_BOX_H * ESZ;
     // every TMA destination (stage start + b * BOX_BYTES) must be 128-byte aligned
     static_assert(BOX_BYTES % 128 == 0 && STAGE_BYTES % 128 == 0, "TMA box / stage not 128-byte aligned");
+    constexpr int W2 = StageGeom<T>::W2, W3 = StageGeom<T>::W3;
+    constexpr int BOX2_BYTES = W2 * ST_BOX_H * ESZ, BOX3_BYTES = W3 * ST_BOX_H * ESZ;
+    static_assert(BOX2_BYTES % 128 == 0 && BOX3_BYTES % 128 == 0 && W2 <= 256 && W3 <= 256, "wide TMA boxes");
+    static_assert(BOX2_BYTES * StageGeom<T>::MAXB2 <= STAGE_BYTES && BOX3_BYTES * StageGeom<T>::MAXB3 <= STAGE_BYTES,
+                  "wide boxes fit the stage");
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
     // TMA destinations must be 128-byte aligned: round the dynamic buffer up (the host
@@ -171,6 +201,7 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__
     uint64_t* empty = full + S;                                                      // S
     float4* partial = reinterpret_cast<float4*>(empty + S);                          // 256 (cluster sum)
     __shared__ mr_grid s_g;
+    __shared__ uint32_t origin_ring[S];
 
     cg::cluster_group cluster = cg::this_cluster();
     const int crank = (int)cluster.block_rank();
@@ -253,7 +284,7 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__
                 const int cnt = min(32, nv - vb);
                 __syncwarp();
                 if (lane < cnt)
-                    meta_new[lane] = view_meta<KIND, T>(views[v_begin + vb + lane], g, ox, oy, oz, di_max,
+                    meta_new[lane] = view_meta<KIND, WIDE, T>(views[v_begin + vb + lane], g, ox, oy, oz, di_max,
                                                         dj_max, R, C);
                 __syncwarp();
                 // lane 0 frees and arms the stage, then lane b issues the copy of box b: the
@@ -266,13 +297,27 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__
                     if (lane == 0) {
                         if (u > 0) mbar_wait(&empty[s], (u - 1) & 1u, status);
                         meta_ring[s] = meta_new[l].rec;
-                        if (mode == MODE_STAGED) mbar_arrive_tx(&full[s], (uint32_t)(nbox * BOX_BYTES));
-                        else mbar_arrive(&full[s]);
+                        if (mode == MODE_STAGED) {
+                            mbar_arrive_tx(&full[s], (uint32_t)(nbox * BOX_BYTES));
+                        } else if (WIDE && (mode == MODE_WIDE2 || mode == MODE_WIDE3)) {
+                            origin_ring[s] = meta_new[l].origin;
+                            mbar_arrive_tx(&full[s], (uint32_t)(nbox * (mode == MODE_WIDE2 ? BOX2_BYTES : BOX3_BYTES)));
+                        } else {
+                            mbar_arrive(&full[s]);
+                        }
                     }
                     __syncwarp();                   // the stage is free and armed for every lane
-                    if (mode == MODE_STAGED && lane < nbox)
-                        tma_load_3d(stages + s * STAGE_BYTES + lane * BOX_BYTES, &tmap, meta_new[l].x0,
+                    if (mode == MODE_STAGED) {
+                        if (lane < nbox)
+                            tma_load_3d(stages + s * STAGE_BYTES + lane * BOX_BYTES, &tmap, meta_new[l].x0,
+                                        meta_new[l].r0 + lane * ST_BOX_H, v_begin + vb + l, &full[s]);
+                    } else if (WIDE && mode == MODE_WIDE2 && lane < nbox) {
+                        tma_load_3d(stages + s * STAGE_BYTES + lane * BOX2_BYTES, &tmap2, meta_new[l].x0,
                                     meta_new[l].r0 + lane * ST_BOX_H, v_begin + vb + l, &full[s]);
+                    } else if (WIDE && mode == MODE_WIDE3 && lane < nbox) {
+                        tma_load_3d(stages + s * STAGE_BYTES + lane * BOX3_BYTES, &tmap3, meta_new[l].x0,
+                                    meta_new[l].r0 + lane * ST_BOX_H, v_begin + vb + l, &full[s]);
+                    }
                 }
             }
         }
@@ -357,6 +402,40 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__
                         const float2 wgt = KIND == MR_CONE ? __fmul2_rn(r, r) : make_float2(m.c.y, m.c.y);
                         acc2[h] = __ffma2_rn(wgt, val, acc2[h]);
                     }
+                } else if (WIDE && (mode == MODE_WIDE2 || mode == MODE_WIDE3)) {
+                    // the global path's arithmetic on taps from a wide box
+                    const uint32_t base = smem_u32(stages + s * STAGE_BYTES);
+                    const uint32_t maxoff = __float_as_uint(m.c.z), kofs = origin_ring[s];
+                    const uint32_t pitch_b = mode == MODE_WIDE2 ? W2 * ESZ : W3 * ESZ;
+#pragma unroll
+                    for (int h = 0; h < ST_PPT / 2; ++h) {
+                        if (!(wlive[2 * h] | wlive[2 * h + 1])) continue;
+                        float2 col = __ffma2_rn(fi2[h], make_float2(m.a.y, m.a.y), make_float2(bu, bu));
+                        float2 row = __ffma2_rn(fi2[h], make_float2(m.b.x, m.b.x), make_float2(bv, bv));
+                        float2 r = make_float2(1.f, 1.f);
+                        if (KIND == MR_CONE) {
+                            const float2 w = __ffma2_rn(fi2[h], make_float2(m.b.w, m.b.w), make_float2(bw, bw));
+                            r = make_float2(rcp_approx(w.x), rcp_approx(w.y));
+                            col = __fmul2_rn(col, r);
+                            row = __fmul2_rn(row, r);
+                        }
+                        const float2 yc = __fadd2_rd(col, kMagic2), yr = __fadd2_rd(row, kMagic2);
+                        const float2 fc = __ffma2_rn(__fadd2_rn(yc, make_float2(-MAGIC, -MAGIC)), kNeg2, col);
+                        const float2 fr = __ffma2_rn(__fadd2_rn(yr, make_float2(-MAGIC, -MAGIC)), kNeg2, row);
+                        const uint32_t a0 = base + min((uint32_t)__float_as_int(yr.x) * pitch_b +
+                                                           (uint32_t)__float_as_int(yc.x) * (uint32_t)ESZ - kofs, maxoff);
+                        const uint32_t a1 = base + min((uint32_t)__float_as_int(yr.y) * pitch_b +
+                                                           (uint32_t)__float_as_int(yc.y) * (uint32_t)ESZ - kofs, maxoff);
+                        const float2 q00 = make_float2(lds_elem<T>(a0), lds_elem<T>(a1));
+                        const float2 q01 = make_float2(lds_elem<T>(a0 + ESZ), lds_elem<T>(a1 + ESZ));
+                        const float2 q10 = make_float2(lds_elem<T>(a0 + pitch_b), lds_elem<T>(a1 + pitch_b));
+                        const float2 q11 = make_float2(lds_elem<T>(a0 + pitch_b + ESZ), lds_elem<T>(a1 + pitch_b + ESZ));
+                        const float2 ta = __ffma2_rn(fc, __ffma2_rn(q00, kNeg2, q01), q00);
+                        const float2 tb = __ffma2_rn(fc, __ffma2_rn(q10, kNeg2, q11), q10);
+                        const float2 val = __ffma2_rn(fr, __ffma2_rn(ta, kNeg2, tb), ta);
+                        const float2 wgt = KIND == MR_CONE ? __fmul2_rn(r, r) : make_float2(m.c.y, m.c.y);
+                        acc2[h] = __ffma2_rn(wgt, val, acc2[h]);
+                    }
                 } else if (mode == MODE_GLOBAL) {
                     const T* q = ring + (long long)(v_begin + v) * slot_stride;
 #pragma unroll
@@ -413,18 +492,20 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__
 }
 
 // ---------------------------------------------------------------- host side
-template <int KIND, typename T>
+template <int KIND, bool WIDE, typename T>
 static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
                          const mr_tile* tiles, int64_t n_tiles, float* out, int* status, cudaStream_t st,
                          const int64_t* n_tiles_dev = nullptr, unsigned int* counter = nullptr) {
-    CUtensorMap map;
+    CUtensorMap map, map2, map3;
     int rc = make_ring_map<T>(ring, StageGeom<T>::W, &map);
+    if (rc == MR_OK) rc = make_ring_map<T>(ring, StageGeom<T>::W2, &map2);
+    if (rc == MR_OK) rc = make_ring_map<T>(ring, StageGeom<T>::W3, &map3);
     if (rc != MR_OK) return rc;
     constexpr int S = StageGeom<T>::STAGES;
     const size_t smem = (size_t)S * StageGeom<T>::W * ST_BOX_H * StageGeom<T>::MAXB * sizeof(T) +
                         S * sizeof(ViewRec) + 32 * sizeof(ViewMeta) + 2 * S * sizeof(uint64_t) +
                         ST_CONSUMERS * 32 * sizeof(float4) + 128;
-    auto kern = bp_staged_kernel<KIND, T>;
+    auto kern = bp_staged_kernel<KIND, WIDE, T>;
     MR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(ST_THREADS);
@@ -446,7 +527,7 @@ static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_gri
         if ((int64_t)clusters > n_tiles) clusters = (int)(n_tiles > 0 ? n_tiles : 1);
         MR_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned int), st));
         cfg.gridDim = dim3((unsigned)(clusters * ST_CLUSTER));
-        MR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, map, static_cast<const T*>(ring->data), ring->rows, ring->cols,
+        MR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, map, map2, map3, static_cast<const T*>(ring->data), ring->rows, ring->cols,
                                        ring->col_pitch, (long long)ring->slot_stride, (int)ring->n_slots, views,
                                        grids, tiles, out, status, n_tiles_dev, counter, (long long)n_tiles));
     } else {
@@ -454,7 +535,7 @@ static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_gri
         for (int64_t t0 = 0; t0 < n_tiles; t0 += max_chunk) {
             const int64_t n = (n_tiles - t0) < max_chunk ? (n_tiles - t0) : max_chunk;
             cfg.gridDim = dim3((unsigned)(n * ST_CLUSTER));
-            MR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, map, static_cast<const T*>(ring->data), ring->rows,
+            MR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, map, map2, map3, static_cast<const T*>(ring->data), ring->rows,
                                            ring->cols, ring->col_pitch, (long long)ring->slot_stride,
                                            (int)ring->n_slots, views, grids, tiles + t0, out, status,
                                            (const int64_t*)nullptr, (unsigned int*)nullptr, (long long)n));
@@ -464,17 +545,19 @@ static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_gri
     return MR_OK;
 }
 
-template <typename... Args>
+template <bool WIDE = false, typename... Args>
 static int dispatch_staged(const mr_ring* ring, Args... args) {
     const bool cone = ring->kind == MR_CONE;
     switch (ring->dtype) {
         case MR_F32:
-            return cone ? launch_staged<MR_CONE, float>(ring, args...) : launch_staged<MR_PARALLEL, float>(ring, args...);
+            return cone ? launch_staged<MR_CONE, WIDE, float>(ring, args...)
+                        : launch_staged<MR_PARALLEL, WIDE, float>(ring, args...);
         case MR_BF16:
-            return cone ? launch_staged<MR_CONE, __nv_bfloat16>(ring, args...)
-                        : launch_staged<MR_PARALLEL, __nv_bfloat16>(ring, args...);
+            return cone ? launch_staged<MR_CONE, WIDE, __nv_bfloat16>(ring, args...)
+                        : launch_staged<MR_PARALLEL, WIDE, __nv_bfloat16>(ring, args...);
         default:
-            return cone ? launch_staged<MR_CONE, __half>(ring, args...) : launch_staged<MR_PARALLEL, __half>(ring, args...);
+            return cone ? launch_staged<MR_CONE, WIDE, __half>(ring, args...)
+                        : launch_staged<MR_PARALLEL, WIDE, __half>(ring, args...);
     }
 }
 
@@ -489,6 +572,18 @@ extern "C" int mr_backproject_staged(const mr_ring* ring, const mr_view* views, 
     if (n_tiles == 0) return MR_OK;
     return mr::dispatch_staged(ring, views, grids, tiles, n_tiles, out, status, static_cast<cudaStream_t>(stream),
                                (const int64_t*)nullptr, (unsigned int*)nullptr);
+}
+
+extern "C" int mr_backproject_staged_wide(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
+                                          const mr_tile* tiles, int64_t n_tiles, float* out, int32_t* status,
+                                          void* stream) {
+    int rc = mr::check_staged_ring(ring);
+    if (rc != MR_OK) return rc;
+    if (!views || !grids || !out || n_tiles < 0 || (n_tiles > 0 && !tiles)) return MR_ERR_INVALID;
+    if (n_tiles == 0) return MR_OK;
+    return mr::dispatch_staged<true>(ring, views, grids, tiles, n_tiles, out, status,
+                                     static_cast<cudaStream_t>(stream), (const int64_t*)nullptr,
+                                     (unsigned int*)nullptr);
 }
 
 extern "C" int mr_backproject_persistent(const mr_ring* ring, const mr_view* views, const mr_grid* grids,

@@ -245,6 +245,13 @@ RAW_LINE_BOUND = 11.1
 # four CTAs, so fewer than 64 leave SMs idle.
 BLOCK_VOLUME_MIN = 64
 
+# Width of a tile's side (31 sample steps) in detector pixels from which a grid goes to
+# mr_backproject_staged_wide. A view sees a square tile 1 to 1.4 sides wide and a stage takes 76
+# pixels, so from about 64 most views exceed it (25 axial 192^2 slices, side 81: 1739 -> 1003 us);
+# below, the few that do are cheaper through global memory (ten 601^2 slices, side 57: 1243 us,
+# 1316 us with the wide variant).
+WIDE_TILE_PIXELS = 64
+
 
 def _device(device=None):
     if not torch.cuda.is_available():
@@ -416,7 +423,7 @@ class KernelTimer:
 
 
 def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, kernel="staged",
-                       status=None, wait=None, asynchronous=False, band_axis=None):
+                       status=None, wait=None, asynchronous=False, band_axis=None, wide_step=None):
     """Back-project numpy GRID_DTYPE records into the device f32 tensor `out`.
 
     kernel="staged": regular grids go through mr_backproject_staged (TMA-staged
@@ -425,7 +432,9 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     wait: an event the launch must follow (the filter of the views summed); the grid and
     tile records are uploaded before the stream waits for it (asynchronously from
     page-locked memory with asynchronous=True). band_axis: the orbit's rotation axis, which
-    orders the tiles of regular grids by height (_native.plan_tiles)."""
+    orders the tiles of regular grids by height (_native.plan_tiles). wide_step: grids with a
+    sample step longer than this across the axis go through mr_backproject_staged_wide (the
+    same result bit for bit; see wide_grids)."""
     grids = np.ascontiguousarray(grids, dtype=N.GRID_DTYPE)
     is_pts = (grids["flags"] & N.MR_GRID_POINTS) != 0
     if kernel == "staged" and is_pts.any() and not is_pts.all():
@@ -434,6 +443,13 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
         wait = None
         grids = grids[~is_pts]
         is_pts = is_pts[~is_pts]
+    wide = wide_grids(grids, band_axis, wide_step) & ((kernel == "staged") & ~is_pts)
+    if wide.any() and not wide.all():
+        backproject_device(ring, views_dev, grids[wide], out, stream, device, timer, kernel, status, wait,
+                           asynchronous, band_axis, wide_step)
+        wait = None
+        grids = grids[~wide]
+        wide = wide[~wide]
     tiles = N.plan_tiles(grids, band_axis)
     if len(tiles) == 0:
         if wait is not None:
@@ -451,10 +467,9 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     name = "mr_backproject_staged" if staged else "mr_backproject"
     ev0 = timer.start(stream) if timer is not None else None
     if staged:
-        st = lib.mr_backproject_staged(ring, v(views_dev.data_ptr()), v(g_ptr), v(t_ptr),
-                                       len(tiles), v(out.data_ptr()),
-                                       v(status.data_ptr()) if status is not None else None,
-                                       v(stream.cuda_stream))
+        fn = lib.mr_backproject_staged_wide if wide.any() else lib.mr_backproject_staged
+        st = fn(ring, v(views_dev.data_ptr()), v(g_ptr), v(t_ptr), len(tiles), v(out.data_ptr()),
+                v(status.data_ptr()) if status is not None else None, v(stream.cuda_stream))
     else:
         st = lib.mr_backproject(ring, v(views_dev.data_ptr()), v(g_ptr), v(t_ptr),
                                 len(tiles), v(out.data_ptr()), v(stream.cuda_stream))
@@ -463,6 +478,18 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     N.check(st, name)
     # keep the descriptor tensor alive until the kernel has consumed it
     recs.record_stream(stream)
+
+
+def wide_grids(grids, band_axis, wide_step):
+    """Which regular grids have tiles whose footprints are mostly wider than a stage of
+    mr_backproject_staged (76 columns): a sample step across the orbit's axis longer than
+    wide_step, WIDE_TILE_PIXELS / 31 detector pixels at the axis."""
+    if band_axis is None or wide_step is None:
+        return np.zeros(len(grids), dtype=bool)
+    a = np.asarray(band_axis, dtype=np.float64)
+    across = lambda s: np.linalg.norm(s - (s @ a)[:, None] * a, axis=1)        # noqa: E731
+    steps = [across(grids[k].astype(np.float64)) for k in ("step_i", "step_j")]
+    return np.maximum(*steps) > wide_step
 
 
 def is_block_volume(grids):
@@ -720,6 +747,7 @@ class SliceReconstructor:
                 print("note: short scan (<360 deg) - no Parker weights, expect some artefacts")
         else:
             raise TypeError(type(geom))
+        self._wide_step = WIDE_TILE_PIXELS / 31 * self.native_pixel
         ramp_response(C, 1.0, window)          # validates the window name early
 
         with torch.cuda.device(self.device):
@@ -1275,6 +1303,9 @@ class SliceReconstructor:
             if len(tiles) == 0:
                 return
             lib = N.load()
+            launch = lib.mr_backproject_staged
+            if wide_grids(grids, self._band_axis, self._wide_step).all():
+                launch = lib.mr_backproject_staged_wide
             v = ctypes_void
             with torch.cuda.device(self.device), torch.cuda.stream(stream):
                 # one upload for all ranges and the tiles; launch i reads its own G records
@@ -1286,10 +1317,9 @@ class SliceReconstructor:
                         stream.wait_event(e)
                     tm = self.kernel_timer
                     ev0 = tm.start(stream) if tm is not None else None
-                    rc = lib.mr_backproject_staged(self._ring_c, v(self._views_dev.data_ptr()),
-                                                   v(g_ptr + i * G * N.GRID_DTYPE.itemsize),
-                                                   v(t_ptr), len(tiles), v(out.data_ptr()), st_ptr,
-                                                   v(stream.cuda_stream))
+                    rc = launch(self._ring_c, v(self._views_dev.data_ptr()),
+                                v(g_ptr + i * G * N.GRID_DTYPE.itemsize), v(t_ptr), len(tiles),
+                                v(out.data_ptr()), st_ptr, v(stream.cuda_stream))
                     if tm is not None:
                         tm.stop("mr_backproject_staged", ev0, stream)
                     N.check(rc, "mr_backproject_staged")
@@ -1301,7 +1331,8 @@ class SliceReconstructor:
             # the copy engines): the records go up without the host waiting
             backproject_device(self._ring_c, self._views_dev, grids, out, stream, self.device,
                                self.kernel_timer, self.bp_kernel, self._status, wait=event,
-                               asynchronous=not self._chunk_marks, band_axis=self._band_axis)
+                               asynchronous=not self._chunk_marks, band_axis=self._band_axis,
+                               wide_step=self._wide_step)
 
     def reconstruct_points_tensor(self, pts, cor_shift=None):
         """Device variant of reconstruct_points: pts (M, 3) -> f32 tensor [M]."""
