@@ -38,22 +38,24 @@ def test_wide_boxes_change_nothing(cuda, store, kind):
     grids["out_offset"] = np.cumsum([0] + [45 * 45] * (len(grids) - 1))
     grids["n_views"], grids["scale"], grids["cor_shift"] = A, np.pi / A, 0.7
     images = []
-    for step in (None, 0.0):                       # no grid, then every grid through the wide variant
+    # no grid, every grid, and two of three (two launches) through the wide variant
+    for wide in (None, [True] * len(grids), [k % 3 > 0 for k in range(len(grids))]):
         out = torch.full((len(grids) * 45 * 45,), float("nan"), dtype=torch.float32, device="cuda")
         status = torch.zeros(1, dtype=torch.int32, device="cuda")
         R.backproject_device(ring.c, ring.views, grids, out, torch.cuda.current_stream(), out.device, status=status,
-                             band_axis=(0.0, 0.0, 1.0), wide_step=step)
+                             band_axis=(0.0, 0.0, 1.0), wide=wide)
         torch.cuda.synchronize()
         assert int(status.item()) == 0
         images.append(out.cpu().numpy())
     assert np.abs(images[0]).max() > 0 and np.isfinite(images[0]).all()
     np.testing.assert_array_equal(images[0], images[1])
+    np.testing.assert_array_equal(images[0], images[2])
 
 
 def test_which_grids_are_wide():
     g = np.zeros(4, N.GRID_DTYPE)
     g["step_i"] = [(0, 1.0, 0), (0, 0.5, 0), (0, 0, 5.0), (0.6, 0.6, 3.0)]
     g["step_j"] = [(0.2, 0, 0), (0.2, 0, 0), (0.2, 0, 0), (0.2, 0, 0)]
-    np.testing.assert_array_equal(R.wide_grids(g, (0.0, 0.0, 1.0), 0.8), [True, False, False, True])
-    np.testing.assert_array_equal(R.wide_grids(g, (0.0, 1.0, 0.0), 0.8), [False, False, True, True])
-    assert not R.wide_grids(g, None, 0.8).any() and not R.wide_grids(g, (0.0, 0.0, 1.0), None).any()
+    assert [R.is_wide(x, (0.0, 0.0, 1.0), 0.8) for x in g] == [True, False, False, True]
+    assert [R.is_wide(x, (0.0, 1.0, 0.0), 0.8) for x in g] == [False, False, True, True]
+    assert not any(R.is_wide(x, None, 0.8) for x in g)

@@ -330,9 +330,9 @@ class _RecordStaging:
             self.host[o:o + n] = raw
             dst = torch.empty(n, dtype=torch.uint8, device=device) if out is None else out
             dst.copy_(self.buf[o:o + n], non_blocking=True)
-            ev = torch.cuda.Event()
-            ev.record(torch.cuda.current_stream(device))
-            self.events[k] = ev
+            if self.events[k] is None:
+                self.events[k] = torch.cuda.Event()
+            self.events[k].record(torch.cuda.current_stream(device))
         return dst
 
 
@@ -423,7 +423,7 @@ class KernelTimer:
 
 
 def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, kernel="staged",
-                       status=None, wait=None, asynchronous=False, band_axis=None, wide_step=None):
+                       status=None, wait=None, asynchronous=False, band_axis=None, wide=None):
     """Back-project numpy GRID_DTYPE records into the device f32 tensor `out`.
 
     kernel="staged": regular grids go through mr_backproject_staged (TMA-staged
@@ -432,9 +432,9 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     wait: an event the launch must follow (the filter of the views summed); the grid and
     tile records are uploaded before the stream waits for it (asynchronously from
     page-locked memory with asynchronous=True). band_axis: the orbit's rotation axis, which
-    orders the tiles of regular grids by height (_native.plan_tiles). wide_step: grids with a
-    sample step longer than this across the axis go through mr_backproject_staged_wide (the
-    same result bit for bit; see wide_grids)."""
+    orders the tiles of regular grids by height (_native.plan_tiles). wide: which grids go
+    through mr_backproject_staged_wide (the same result bit for bit; see is_wide), one truth
+    value each, or None for none."""
     grids = np.ascontiguousarray(grids, dtype=N.GRID_DTYPE)
     is_pts = (grids["flags"] & N.MR_GRID_POINTS) != 0
     if kernel == "staged" and is_pts.any() and not is_pts.all():
@@ -443,13 +443,14 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
         wait = None
         grids = grids[~is_pts]
         is_pts = is_pts[~is_pts]
-    wide = wide_grids(grids, band_axis, wide_step) & ((kernel == "staged") & ~is_pts)
-    if wide.any() and not wide.all():
-        backproject_device(ring, views_dev, grids[wide], out, stream, device, timer, kernel, status, wait,
-                           asynchronous, band_axis, wide_step)
-        wait = None
-        grids = grids[~wide]
-        wide = wide[~wide]
+    all_wide = wide is not None and kernel == "staged" and len(grids) > 0 and not is_pts.any() and all(wide)
+    if not all_wide and wide is not None and kernel == "staged" and not is_pts.any() and any(wide):
+        w = np.asarray(wide, dtype=bool)
+        for part, flag in ((grids[w], [True] * int(w.sum())), (grids[~w], None)):
+            backproject_device(ring, views_dev, part, out, stream, device, timer, kernel, status, wait, asynchronous,
+                               band_axis, flag)
+            wait = None
+        return
     tiles = N.plan_tiles(grids, band_axis)
     if len(tiles) == 0:
         if wait is not None:
@@ -467,7 +468,7 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     name = "mr_backproject_staged" if staged else "mr_backproject"
     ev0 = timer.start(stream) if timer is not None else None
     if staged:
-        fn = lib.mr_backproject_staged_wide if wide.any() else lib.mr_backproject_staged
+        fn = lib.mr_backproject_staged_wide if all_wide else lib.mr_backproject_staged
         st = fn(ring, v(views_dev.data_ptr()), v(g_ptr), v(t_ptr), len(tiles), v(out.data_ptr()),
                 v(status.data_ptr()) if status is not None else None, v(stream.cuda_stream))
     else:
@@ -480,16 +481,19 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     recs.record_stream(stream)
 
 
-def wide_grids(grids, band_axis, wide_step):
-    """Which regular grids have tiles whose footprints are mostly wider than a stage of
-    mr_backproject_staged (76 columns): a sample step across the orbit's axis longer than
+def is_wide(grid, band_axis, wide_step):
+    """Whether the tiles of a regular grid (one record) have footprints mostly wider than a stage
+    of mr_backproject_staged (76 columns): a sample step across the orbit's axis longer than
     wide_step, WIDE_TILE_PIXELS / 31 detector pixels at the axis."""
-    if band_axis is None or wide_step is None:
-        return np.zeros(len(grids), dtype=bool)
-    a = np.asarray(band_axis, dtype=np.float64)
-    across = lambda s: np.linalg.norm(s - (s @ a)[:, None] * a, axis=1)        # noqa: E731
-    steps = [across(grids[k].astype(np.float64)) for k in ("step_i", "step_j")]
-    return np.maximum(*steps) > wide_step
+    if band_axis is None:
+        return False
+    a = [float(x) for x in band_axis]
+    for k in ("step_i", "step_j"):
+        s = grid[k].tolist()
+        along = sum(x * y for x, y in zip(s, a))
+        if sum(x * x for x in s) - along * along > wide_step * wide_step:
+            return True
+    return False
 
 
 def is_block_volume(grids):
@@ -1271,24 +1275,24 @@ class SliceReconstructor:
         with self._lock:
             return self.n, self.cor_shift, self._ingest_event
 
-    def _run_grids(self, grids, out, n, event):
+    def _run_grids(self, grids, out, n, event, wide=None):
         """Launch the batched back-projection of `grids` into device `out`. Right after a
         chunked host upload, the views are summed chunk by chunk: each partial launch
         waits only for its own chunk's filter, so the reconstruction overlaps the transfer
-        of the later chunks (same scale; FP32 partial sums added in view order)."""
+        of the later chunks (same scale; FP32 partial sums added in view order). Called with the
+        device and the reconstruction stream current. wide: see backproject_device."""
         stream = self.stream
         grids["scale"] = np.pi / n if n else 0.0
         marks = [(se, e) for se, e in self._chunk_marks if 0 < se < n]
         regular = not (np.asarray(grids["flags"]) & N.MR_GRID_POINTS).any()
         if self.bp_kernel == "staged" and is_block_volume(grids):
             bounds = [0] + [se for se, _ in marks] + [n]
-            with torch.cuda.device(self.device):
-                for a, b, e in zip(bounds[:-1], bounds[1:], [e for _, e in marks] + [event]):
-                    if e is not None:
-                        stream.wait_event(e)
-                    grids["view_begin"], grids["n_views"], grids["accumulate"] = a, b - a, int(a > 0)
-                    backproject_volume_device(self._ring_c, self._views_dev, grids, out, stream,
-                                              self.kernel_timer, self._status)
+            for a, b, e in zip(bounds[:-1], bounds[1:], [e for _, e in marks] + [event]):
+                if e is not None:
+                    stream.wait_event(e)
+                grids["view_begin"], grids["n_views"], grids["accumulate"] = a, b - a, int(a > 0)
+                backproject_volume_device(self._ring_c, self._views_dev, grids, out, stream, self.kernel_timer,
+                                          self._status)
             return
         if marks and regular and self.bp_kernel == "staged":
             bounds = [0] + [se for se, _ in marks] + [n]
@@ -1303,9 +1307,7 @@ class SliceReconstructor:
             if len(tiles) == 0:
                 return
             lib = N.load()
-            launch = lib.mr_backproject_staged
-            if wide_grids(grids, self._band_axis, self._wide_step).all():
-                launch = lib.mr_backproject_staged_wide
+            launch = lib.mr_backproject_staged_wide if wide and all(wide) else lib.mr_backproject_staged
             v = ctypes_void
             with torch.cuda.device(self.device), torch.cuda.stream(stream):
                 # one upload for all ranges and the tiles; launch i reads its own G records
@@ -1326,13 +1328,11 @@ class SliceReconstructor:
                 recs.record_stream(stream)
             return
         grids["n_views"] = n
-        with torch.cuda.device(self.device), torch.cuda.stream(stream):
-            # no chunked host upload in flight (it would sit ahead of a page-locked copy on
-            # the copy engines): the records go up without the host waiting
-            backproject_device(self._ring_c, self._views_dev, grids, out, stream, self.device,
-                               self.kernel_timer, self.bp_kernel, self._status, wait=event,
-                               asynchronous=not self._chunk_marks, band_axis=self._band_axis,
-                               wide_step=self._wide_step)
+        # no chunked host upload in flight (it would sit ahead of a page-locked copy on
+        # the copy engines): the records go up without the host waiting
+        backproject_device(self._ring_c, self._views_dev, grids, out, stream, self.device,
+                           self.kernel_timer, self.bp_kernel, self._status, wait=event,
+                           asynchronous=not self._chunk_marks, band_axis=self._band_axis, wide=wide)
 
     def reconstruct_points_tensor(self, pts, cor_shift=None):
         """Device variant of reconstruct_points: pts (M, 3) -> f32 tensor [M]."""
@@ -1365,41 +1365,56 @@ class SliceReconstructor:
         shift = self.cor_shift if cor_shift is None else float(cor_shift)
         return plane_grid(self.box, origin, normal, int(n), size, zoom, center, shift)
 
-    def _plane_record(self, origin, normal, n, size, zoom, center, shift):
-        """plane_grid for this reconstructor's box, memoised on the request's parameters
-        (the FP64 plane set-up is pure; a repeated request skips it on the host)."""
-        flat = lambda v: None if v is None else tuple(float(x) for x in np.ravel(v))   # noqa: E731
-        key = (flat(origin), flat(normal), int(n), None if size is None else float(size), float(zoom),
-               flat(center), float(shift))
+    def _plane_entry(self, origin, normal, n, size, zoom, center, shift):
+        """(record bytes, wide) of plane_grid for this reconstructor's box, memoised on the
+        request's parameters (the FP64 plane set-up is pure; a repeated request skips it on the
+        host). wide: see is_wide."""
+        scale = (n, None if size is None else float(size), float(zoom), float(shift))
+        try:
+            key = (tuple(map(float, origin)), tuple(map(float, normal)),
+                   None if center is None else tuple(map(float, center)), scale)
+        except TypeError:                                   # nested sequences
+            flat = lambda v: None if v is None else tuple(float(x) for x in np.ravel(v))   # noqa: E731
+            key = (flat(origin), flat(normal), flat(center), scale)
         cache = self.__dict__.setdefault("_plane_cache", collections.OrderedDict())
-        rec = cache.get(key)
-        if rec is None:
+        entry = cache.get(key)
+        if entry is None:
             rec = plane_grid(self.box, origin, normal, n, size, zoom, center, shift)
-            cache[key] = rec
+            entry = (rec.tobytes(), is_wide(rec, self._band_axis, self._wide_step))
+            cache[key] = entry
             if len(cache) > 256:
                 cache.popitem(last=False)
         else:
             cache.move_to_end(key)
-        return rec.copy()
+        return entry
+
+    def _plane_record(self, origin, normal, n, size, zoom, center, shift):
+        """The mr_grid record of _plane_entry."""
+        rec = self._plane_entry(origin, normal, int(n), size, zoom, center, shift)[0]
+        return np.frombuffer(bytearray(rec), dtype=N.GRID_DTYPE)[0]
 
     def _planes(self, requests):
         """One batched launch for many slices -> (flat f32 device tensor, sizes)."""
         n_views, shift, ev = self._snapshot()
-        grids = np.zeros(len(requests), dtype=N.GRID_DTYPE)
-        sizes, offset = [], 0
-        for r, req in enumerate(requests):
-            n = int(req.get("n", 256))
-            s_ = req.get("cor_shift")
-            grids[r] = self._plane_record(req["origin"], req["normal"], n, req.get("size"),
-                                          req.get("zoom", 1.0), req.get("center"),
-                                          shift if s_ is None else float(s_))
-            grids[r]["out_offset"] = offset
+        entries, sizes, offsets, offset = [], [], [], 0
+        for req in requests:
+            get = req.get
+            n = int(get("n", 256))
+            s_ = get("cor_shift")
+            entries.append(self._plane_entry(req["origin"], req["normal"], n, get("size"), get("zoom", 1.0),
+                                             get("center"), shift if s_ is None else float(s_)))
+            offsets.append(offset)
             sizes.append(n)
             offset += n * n
+        grids = np.frombuffer(bytearray(b"".join([e[0] for e in entries])), dtype=N.GRID_DTYPE)
+        grids["out_offset"] = offsets
         with torch.cuda.device(self.device), torch.cuda.stream(self.stream):
-            out = torch.zeros(offset, dtype=torch.float32, device=self.device)
             if n_views > 0 and offset > 0:
-                self._run_grids(grids, out, n_views, ev)
+                # every sample of every grid is written, those outside the box as 0
+                out = torch.empty(offset, dtype=torch.float32, device=self.device)
+                self._run_grids(grids, out, n_views, ev, [e[1] for e in entries])
+            else:
+                out = torch.zeros(offset, dtype=torch.float32, device=self.device)
         _handoff(self.stream, out)
         return out, sizes
 
