@@ -17,6 +17,7 @@
 // Each warp covers compact 8 (j) x 4 (i) sample patches so its LDS gathers touch a small
 // 2D patch (few bank conflicts) for any plane orientation.
 #include <cooperative_groups.h>
+#include <cmath>
 
 #include "bp_stage.cuh"
 
@@ -25,9 +26,19 @@ namespace cg = cooperative_groups;
 namespace mr {
 
 constexpr int ST_TI = 32, ST_TJ = 32;        // tile (samples) - same tiling as bp.cu
-constexpr int ST_CONSUMERS = 8;               // consumer warps (one 32 x 32 tile)
-constexpr int ST_THREADS = 32 * (ST_CONSUMERS + 1);   // + one producer warp
-constexpr int ST_PPT = 4;                     // samples per consumer thread (rows i, i+2, i+4, i+6)
+// Consumer warps of a 32 x 32 tile, and one producer warp. SLIM: half the warps with twice the
+// samples each, which share a view's records and waits and run interleaved, and two stages, so
+// that five CTAs fit an SM (four of FP32); for launches with tiles to fill them (slim_pays).
+// Three 512^2 slices, 600 views, BF16: 508 -> 462 us; one 1024^2 slice 990 -> 876 us; ten 601^2
+// slices of 160 full-resolution views, FP32: 1242 -> 1217 us. Three stages and four CTAs an SM:
+// 459, 819 and 1290 us; a ring of footprint-sized pieces in the place of fixed stages: 518 and
+// 910 us (its bookkeeping is in the producer's path, which the consumers wait for).
+template <bool SLIM> struct Shape {
+    static constexpr int CONSUMERS = SLIM ? 4 : 8;
+    static constexpr int THREADS = 32 * (CONSUMERS + 1);
+    static constexpr int PPT = 32 / CONSUMERS;    // samples per consumer thread (rows i, i+2, ..)
+    static constexpr int CTAS = SLIM ? 5 : 3;     // an SM's, for the register bound
+};
 constexpr int ST_DI = 2;                      // row step between a thread's samples
 constexpr int ST_CLUSTER = 4;                 // CTAs per tile, each a quarter of the views
 
@@ -169,8 +180,8 @@ __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g
 // (DSMEM) in rank order - deterministic, no atomics, no scratch - and writes the tile.
 // Three CTAs fit an SM (shared memory); the launch bound says so, or ptxas aims at four and
 // spills the FP32 variant to fit its registers.
-template <int KIND, bool WIDE, typename T>
-__global__ void __launch_bounds__(ST_THREADS, 3)
+template <int KIND, bool WIDE, bool SLIM, typename T>
+__global__ void __launch_bounds__(Shape<SLIM>::THREADS, Shape<SLIM>::CTAS)
 bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap2,
                  const __grid_constant__ CUtensorMap tmap3, const T* __restrict__ ring, int R, int C,
                  int pitch, long long slot_stride, int n_slots, const mr_view* __restrict__ views,
@@ -178,7 +189,8 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
                  float* __restrict__ out, int* status, const int64_t* __restrict__ n_tiles_dev,
                  unsigned int* __restrict__ counter, long long tile_cap) {
     constexpr int W = StageGeom<T>::W;
-    constexpr int S = StageGeom<T>::STAGES;
+    constexpr int ST_CONSUMERS = Shape<SLIM>::CONSUMERS, ST_PPT = Shape<SLIM>::PPT;
+    constexpr int S = SLIM ? 2 : StageGeom<T>::STAGES;
     constexpr int ESZ = (int)sizeof(T);
     constexpr int STAGE_BYTES = W * ST_BOX_H * StageGeom<T>::MAXB * ESZ;
     constexpr int BOX_BYTES = W * ST_BOX_H * ESZ;
@@ -199,7 +211,7 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
     ViewMeta* meta_new = reinterpret_cast<ViewMeta*>(meta_ring + S);                // 32
     uint64_t* full = reinterpret_cast<uint64_t*>(meta_new + 32);                    // S
     uint64_t* empty = full + S;                                                      // S
-    float4* partial = reinterpret_cast<float4*>(empty + S);                          // 256 (cluster sum)
+    float4* partial = reinterpret_cast<float4*>(empty + S);                          // cluster sum: 1024 floats
     __shared__ mr_grid s_g;
     __shared__ uint32_t origin_ring[S];
 
@@ -254,13 +266,13 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
         const float ox = g.origin[0] + t.i0 * g.step_i[0] + t.j0 * g.step_j[0] + t.k * g.step_k[0];
         const float oy = g.origin[1] + t.i0 * g.step_i[1] + t.j0 * g.step_j[1] + t.k * g.step_k[1];
         const float oz = g.origin[2] + t.i0 * g.step_i[2] + t.j0 * g.step_j[2] + t.k * g.step_k[2];
-        // warp w covers columns 16 (w & 1) .. + 15 and rows 8 (w >> 1) .. + 7 of the tile; its
+        // warp w covers columns 16 (w & 1) .. + 15 and 8 (SLIM: 16) rows from those of w >> 1; its
         // p-th sample step is a 16 x 2 patch (rows ty + 2p). The patch shape keeps the 32
         // lanes' bilinear taps on distinct shared-memory banks for most plane orientations
         // (1.10 wavefronts per 16-bit tap load on the bench slices, 1.35 for 8 x 4 patches)
         // and makes each half-warp's output a 64-byte row segment.
         const int tx = ((warp & 1) << 4) | (lane & 15);
-        const int ty = ((warp >> 1) << 3) | (lane >> 4);
+        const int ty = (warp >> 1) * (2 * ST_PPT) + (lane >> 4);
         bool inside[ST_PPT];
         bool any = false;
 #pragma unroll
@@ -272,10 +284,14 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
             any |= ok;
         }
         const bool tile_live = __syncthreads_or(any) != 0;
-        // warp-uniform: an 8x4 sample patch wholly outside the box is not computed
-        bool wlive[ST_PPT];
+        // warp-uniform: a 16 x 2 sample patch wholly outside the box is not computed. SLIM: only
+        // if all of the warp's are (a branch per pair keeps the pairs from running interleaved)
+        bool wlive[ST_PPT], wany = false;
 #pragma unroll
-        for (int p = 0; p < ST_PPT; ++p) wlive[p] = __any_sync(0xffffffffu, inside[p]);
+        for (int p = 0; p < ST_PPT; ++p) {
+            wlive[p] = __any_sync(0xffffffffu, inside[p]);
+            wany |= wlive[p];
+        }
 
         if (producer && tile_live) {
             const int di_max = min(ST_TI, g.n_i - t.i0) - 1;
@@ -341,7 +357,7 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
                 const float bu = fmaf(fj, m.a.z, m.a.x);
                 const float bv = fmaf(fj, m.b.y, m.a.w);
                 const float bw = fmaf(fj, m.c.x, m.b.z);
-                if (mode == MODE_STAGED) {
+                if (mode == MODE_STAGED && (!SLIM || wany)) {
                     const uint32_t base = smem_u32(stages + s * STAGE_BYTES);
                     const uint32_t maxoff = __float_as_uint(m.c.z);
                     // byte offset = (bits_r - MAGIC_BITS) * W*ESZ + (bits_c - MAGIC_BITS) * ESZ
@@ -354,7 +370,7 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
                     const float2 bu2 = make_float2(bu, bu), bv2 = make_float2(bv, bv), bw2 = make_float2(bw, bw);
 #pragma unroll
                     for (int h = 0; h < ST_PPT / 2; ++h) {
-                        if (!(wlive[2 * h] | wlive[2 * h + 1])) continue;
+                        if (!SLIM && !(wlive[2 * h] | wlive[2 * h + 1])) continue;
                         const float2 nu = __ffma2_rn(fi2[h], cuy, bu2);
                         const float2 nv2 = __ffma2_rn(fi2[h], cvy, bv2);
                         float2 r = make_float2(1.f, 1.f), yc, yr, fc, fr;
@@ -464,14 +480,24 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
         if (tile_live) used += (uint32_t)nv;
 
         // ---- cluster reduction of the view-quarter partial sums (rank order), rank 0 writes
-        float acc[ST_PPT] = {acc2[0].x, acc2[0].y, acc2[1].x, acc2[1].y};
+        float acc[ST_PPT];
+#pragma unroll
+        for (int p = 0; p < ST_PPT; ++p) acc[p] = (p & 1) ? acc2[p >> 1].y : acc2[p >> 1].x;
         if (csize > 1) {
-            if (!producer) partial[tid] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            if (!producer) {
+#pragma unroll
+                for (int q = 0; q < ST_PPT / 4; ++q)
+                    partial[q * (32 * ST_CONSUMERS) + tid] =
+                        make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+            }
             cluster.sync();
             if (crank == 0 && !producer) {
                 for (int r = 1; r < csize; ++r) {
-                    const float4 o = cluster.map_shared_rank(partial, r)[tid];
-                    acc[0] += o.x; acc[1] += o.y; acc[2] += o.z; acc[3] += o.w;
+#pragma unroll
+                    for (int q = 0; q < ST_PPT / 4; ++q) {
+                        const float4 o = cluster.map_shared_rank(partial, r)[q * (32 * ST_CONSUMERS) + tid];
+                        acc[4 * q] += o.x; acc[4 * q + 1] += o.y; acc[4 * q + 2] += o.z; acc[4 * q + 3] += o.w;
+                    }
                 }
             }
         }
@@ -492,7 +518,7 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
 }
 
 // ---------------------------------------------------------------- host side
-template <int KIND, bool WIDE, typename T>
+template <int KIND, bool WIDE, bool SLIM, typename T>
 static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
                          const mr_tile* tiles, int64_t n_tiles, float* out, int* status, cudaStream_t st,
                          const int64_t* n_tiles_dev = nullptr, unsigned int* counter = nullptr) {
@@ -501,14 +527,14 @@ static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_gri
     if (rc == MR_OK) rc = make_ring_map<T>(ring, StageGeom<T>::W2, &map2);
     if (rc == MR_OK) rc = make_ring_map<T>(ring, StageGeom<T>::W3, &map3);
     if (rc != MR_OK) return rc;
-    constexpr int S = StageGeom<T>::STAGES;
+    constexpr int S = SLIM ? 2 : StageGeom<T>::STAGES;
     const size_t smem = (size_t)S * StageGeom<T>::W * ST_BOX_H * StageGeom<T>::MAXB * sizeof(T) +
                         S * sizeof(ViewRec) + 32 * sizeof(ViewMeta) + 2 * S * sizeof(uint64_t) +
-                        ST_CONSUMERS * 32 * sizeof(float4) + 128;
-    auto kern = bp_staged_kernel<KIND, WIDE, T>;
+                        ST_TI * ST_TJ * sizeof(float) + 128;
+    auto kern = bp_staged_kernel<KIND, WIDE, SLIM, T>;
     MR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(ST_THREADS);
+    cfg.blockDim = dim3(Shape<SLIM>::THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -545,19 +571,36 @@ static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_gri
     return MR_OK;
 }
 
-template <bool WIDE = false, typename... Args>
+// Whether a launch of n tiles is faster with SLIM: its CTAs take 1.47 (FP32: 1.24) times as long,
+// but 5/3 (4/3) as many run at once. A launch of x waves costs between x and the next whole
+// number of them; half way between is taken (one slice, 600 views, BF16, full / slim: 64 tiles
+// 340 / 602 us, 144 tiles 196 / 150, 256 tiles 284 / 256, 300 tiles 323 / 305, 625 tiles 597 /
+// 540; FP32, 300 tiles 324 / 362, 256 tiles 283 / 265).
+static bool slim_pays(int64_t n, bool fp32) {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 148;
+    auto cost = [&](int ctas, double time) {
+        const double x = (double)n * ST_CLUSTER / ((double)sms * ctas);
+        return 0.5 * (x + ceil(x)) * time;
+    };
+    return cost(fp32 ? 4 : 5, fp32 ? 1.24 : 1.47) < cost(3, 1.0);
+}
+
+template <bool WIDE, bool SLIM, typename... Args>
 static int dispatch_staged(const mr_ring* ring, Args... args) {
     const bool cone = ring->kind == MR_CONE;
     switch (ring->dtype) {
         case MR_F32:
-            return cone ? launch_staged<MR_CONE, WIDE, float>(ring, args...)
-                        : launch_staged<MR_PARALLEL, WIDE, float>(ring, args...);
+            return cone ? launch_staged<MR_CONE, WIDE, SLIM, float>(ring, args...)
+                        : launch_staged<MR_PARALLEL, WIDE, SLIM, float>(ring, args...);
         case MR_BF16:
-            return cone ? launch_staged<MR_CONE, WIDE, __nv_bfloat16>(ring, args...)
-                        : launch_staged<MR_PARALLEL, WIDE, __nv_bfloat16>(ring, args...);
+            return cone ? launch_staged<MR_CONE, WIDE, SLIM, __nv_bfloat16>(ring, args...)
+                        : launch_staged<MR_PARALLEL, WIDE, SLIM, __nv_bfloat16>(ring, args...);
         default:
-            return cone ? launch_staged<MR_CONE, WIDE, __half>(ring, args...)
-                        : launch_staged<MR_PARALLEL, WIDE, __half>(ring, args...);
+            return cone ? launch_staged<MR_CONE, WIDE, SLIM, __half>(ring, args...)
+                        : launch_staged<MR_PARALLEL, WIDE, SLIM, __half>(ring, args...);
     }
 }
 
@@ -570,8 +613,14 @@ extern "C" int mr_backproject_staged(const mr_ring* ring, const mr_view* views, 
     if (rc != MR_OK) return rc;
     if (!views || !grids || !out || n_tiles < 0 || (n_tiles > 0 && !tiles)) return MR_ERR_INVALID;
     if (n_tiles == 0) return MR_OK;
-    return mr::dispatch_staged(ring, views, grids, tiles, n_tiles, out, status, static_cast<cudaStream_t>(stream),
-                               (const int64_t*)nullptr, (unsigned int*)nullptr);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t* no_count = nullptr;
+    unsigned int* no_counter = nullptr;
+    return mr::slim_pays(n_tiles, ring->dtype == MR_F32)
+               ? mr::dispatch_staged<false, true>(ring, views, grids, tiles, n_tiles, out, status, st, no_count,
+                                                  no_counter)
+               : mr::dispatch_staged<false, false>(ring, views, grids, tiles, n_tiles, out, status, st, no_count,
+                                                   no_counter);
 }
 
 extern "C" int mr_backproject_staged_wide(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
@@ -581,7 +630,7 @@ extern "C" int mr_backproject_staged_wide(const mr_ring* ring, const mr_view* vi
     if (rc != MR_OK) return rc;
     if (!views || !grids || !out || n_tiles < 0 || (n_tiles > 0 && !tiles)) return MR_ERR_INVALID;
     if (n_tiles == 0) return MR_OK;
-    return mr::dispatch_staged<true>(ring, views, grids, tiles, n_tiles, out, status,
+    return mr::dispatch_staged<true, false>(ring, views, grids, tiles, n_tiles, out, status,
                                      static_cast<cudaStream_t>(stream), (const int64_t*)nullptr,
                                      (unsigned int*)nullptr);
 }
@@ -595,7 +644,7 @@ extern "C" int mr_backproject_persistent(const mr_ring* ring, const mr_view* vie
     // the 32-bit work counter must not wrap while the last clusters overshoot the count
     if (max_tiles > (int64_t(1) << 31)) return MR_ERR_INVALID;
     if ((reinterpret_cast<uintptr_t>(counter_dev) & 3) != 0) return MR_ERR_INVALID;
-    return mr::dispatch_staged(ring, views, grids, tiles, max_tiles, out, status, static_cast<cudaStream_t>(stream),
+    return mr::dispatch_staged<false, false>(ring, views, grids, tiles, max_tiles, out, status, static_cast<cudaStream_t>(stream),
                                n_tiles_dev, reinterpret_cast<unsigned int*>(counter_dev));
 }
 
@@ -656,6 +705,6 @@ extern "C" int mr_backproject_persistent_noalloc(const mr_ring* ring, const mr_v
     rc = noalloc_counter(static_cast<cudaStream_t>(stream), &counter);
     if (rc != MR_OK) return rc;
     // the shared launch path zeroes the counter on `stream` before the kernel
-    return mr::dispatch_staged(ring, views, grids, tiles, max_tiles, out, status, static_cast<cudaStream_t>(stream),
+    return mr::dispatch_staged<false, false>(ring, views, grids, tiles, max_tiles, out, status, static_cast<cudaStream_t>(stream),
                                n_tiles_dev, counter);
 }
