@@ -629,7 +629,12 @@ __global__ void __launch_bounds__(256, 2) fft_filter_kernel(Filter2Args A, int s
 #pragma unroll
                 for (int q = 0; q < 16; ++q) {
                     const int c = j + G * q;
-                    if (c < A.pitch) {
+                    if (two && G * (q + 1) <= C) {
+                        // columns inside the row for every thread: no checks (96 views of
+                        // 1944 x 1536: 2142 -> 2117 us)
+                        o[c] = ring_cvt(o, x[q].x);
+                        o[c + A.pitch] = ring_cvt(o, -x[q].y);
+                    } else if (c < A.pitch) {
                         o[c] = ring_cvt(o, c < C ? x[q].x : 0.f);
                         if (two) o[c + A.pitch] = ring_cvt(o, c < C ? -x[q].y : 0.f);
                     }
