@@ -6,15 +6,24 @@
 //   gaussian_blur      preprocess.py:8-28: per axis, edge padding by pad = ceil(3 sigma),
 //       circular convolution of length N = n + 2 pad with g = irfft(exp(-2 (pi f sigma)^2)),
 //       crop. The caller passes g[0..K] (g is even; |m| > K contributes < 1e-20).
+#include <type_traits>
+
 #include "mr_common.cuh"
 
 namespace mr {
 
-__global__ void rotate_kernel(const float* __restrict__ in, float* __restrict__ out, int R, int A,
-                              int C, float ct, float st) {
+// Where an output samples its view, and with what weights, is the same in every view: a thread
+// forms both once for RT_VIEWS views and has the taps of all of them in flight, where a thread of
+// one output waited for its four loads alone (486 x 384, 0.3 degrees: 600 views 483 -> 227 us,
+// 64 views 57 -> 32 us, 8 views 12 -> 10 us, one view 8 us as before; 16 views of 1944 x 1536
+// 209 -> 94 us; the same outputs). A read and a write of the 600 views take 137 us: bound by the
+// four loads an output through L1.
+constexpr int RT_VIEWS = 8;
+__global__ void __launch_bounds__(128) rotate_kernel(const float* __restrict__ in, float* __restrict__ out, int R,
+                                                     int A, int C, float ct, float st) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y;
-    const int a = blockIdx.z;
+    const int a0 = blockIdx.z * RT_VIEWS;
     if (c >= C) return;
     const float rr = (float)r - 0.5f * (float)(R - 1);
     const float cc = (float)c - 0.5f * (float)(C - 1);
@@ -24,19 +33,37 @@ __global__ void rotate_kernel(const float* __restrict__ in, float* __restrict__ 
     const float fr = rs - r0f, fc = cs - c0f;
     const int r0 = (int)r0f, c0 = (int)c0f;
     const long long srow = (long long)A * C;
-    float acc = 0.f;
+    float w[4];
+    bool ok[4];
+    const float* p[4];
 #pragma unroll
-    for (int dr = 0; dr < 2; ++dr) {
-#pragma unroll
-        for (int dc = 0; dc < 2; ++dc) {
-            const int ri = r0 + dr, ci = c0 + dc;
-            if ((unsigned)ri < (unsigned)R && (unsigned)ci < (unsigned)C) {
-                const float w = (dr ? fr : 1.f - fr) * (dc ? fc : 1.f - fc);
-                acc = fmaf(w, __ldg(in + ri * srow + (long long)a * C + ci), acc);
-            }
-        }
+    for (int t = 0; t < 4; ++t) {
+        const int ri = r0 + (t >> 1), ci = c0 + (t & 1);
+        w[t] = (t >> 1 ? fr : 1.f - fr) * (t & 1 ? fc : 1.f - fc);
+        ok[t] = (unsigned)ri < (unsigned)R && (unsigned)ci < (unsigned)C;
+        p[t] = in + (ok[t] ? ri * srow + (long long)a0 * C + ci : 0);
     }
-    out[r * srow + (long long)a * C + c] = acc;
+    float* o = out + r * srow + (long long)a0 * C + c;
+    auto views = [&](int a, auto n) {               // views a0 + a .. a0 + a + n - 1
+        constexpr int V = decltype(n)::value;
+        float x[V][4];
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int t = 0; t < 4; ++t) x[v][t] = ok[t] ? __ldg(p[t] + (long long)(a + v) * C) : 0.f;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            float acc = 0.f;
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (ok[t]) acc = fmaf(w[t], x[v][t], acc);
+            o[(long long)(a + v) * C] = acc;
+        }
+    };
+    const int n = min(RT_VIEWS, A - a0);
+    if (n == RT_VIEWS) views(0, std::integral_constant<int, RT_VIEWS>{});
+    else
+        for (int a = 0; a < n; ++a) views(a, std::integral_constant<int, 1>{});
 }
 
 // One axis of the edge-padded circular Gaussian: along rows (axis 0) or cols (axis 2).
@@ -215,7 +242,7 @@ extern "C" int mr_rotate_f32(const float* in, float* out, int32_t rows, int32_t 
     if (k == 0) return MR_OK;
     const double t = degrees * 3.14159265358979323846 / 180.0;
     const dim3 block(128);
-    const dim3 grid((cols + 127) / 128, rows, k);
+    const dim3 grid((cols + 127) / 128, rows, (k + mr::RT_VIEWS - 1) / mr::RT_VIEWS);
     if (k > 65535 || rows > 65535) return MR_ERR_INVALID;
     mr::rotate_kernel<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(
         in, out, rows, k, cols, (float)cos(t), (float)sin(t));
