@@ -16,8 +16,8 @@ namespace mr {
 // forms both once for RT_VIEWS views and has the taps of all of them in flight, where a thread of
 // one output waited for its four loads alone (486 x 384, 0.3 degrees: 600 views 483 -> 227 us,
 // 64 views 57 -> 32 us, 8 views 12 -> 10 us, one view 8 us as before; 16 views of 1944 x 1536
-// 209 -> 94 us; the same outputs). A read and a write of the 600 views take 137 us: bound by the
-// four loads an output through L1.
+// 209 -> 94 us; the same outputs). A read and a write of the 600 views take 137 us; what is left
+// is latency and issue (63 %) of the four loads an output.
 constexpr int RT_VIEWS = 8;
 __global__ void __launch_bounds__(128) rotate_kernel(const float* __restrict__ in, float* __restrict__ out, int R,
                                                      int A, int C, float ct, float st) {
