@@ -184,6 +184,12 @@ int mr_backproject_staged_wide(const mr_ring* ring, const mr_view* views_dev,
 int mr_backproject_volume(const mr_ring* ring, const mr_view* views_dev, const mr_grid* grid_host,
                           float* out_dev, int32_t* status_dev, void* stream);
 
+/* The same for grids whose voxels are several detector pixels wide: footprints of a block up to
+ * 124 columns x 124 rows (92 of an FP32 ring) are staged, where mr_backproject_volume, whose
+ * stages hold 76 x 60, reads global memory. */
+int mr_backproject_volume_coarse(const mr_ring* ring, const mr_view* views_dev, const mr_grid* grid_host,
+                                 float* out_dev, int32_t* status_dev, void* stream);
+
 /* Persistent form of mr_backproject_staged for serving: a fixed grid of CTA clusters
  * (as many as fit on the GPU at once, at most max_tiles) pulls tile indices from a work
  * counter until it reaches min(*n_tiles_dev, max_tiles) (device int64; max_tiles <= 2^31),

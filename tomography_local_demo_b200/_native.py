@@ -64,6 +64,7 @@ SIGNATURES = {
     "mr_backproject_staged": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P, _P]),
     "mr_backproject_staged_wide": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P, _P]),
     "mr_backproject_volume": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _P]),
+    "mr_backproject_volume_coarse": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _P]),
     "mr_backproject_persistent": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _I64, _P, _P, _P, _P]),
     "mr_backproject_persistent_noalloc": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _I64, _P, _P, _P]),
     "mr_backproject_matched": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P]),

@@ -13,8 +13,8 @@
 // full projection per voxel, and footprints wider than a stage read global memory.
 //
 // Measured (600 views of 486 x 384, against the staged kernel's tiles): 256 x 256 x 203
-// voxels, BF16 ring, 16.9 -> 6.2 ms (1290 G updates/s); FP32 ring, whose tile footprints
-// there did not fit a stage, 52.5 -> 6.6 ms; 400 x 400 x 317 voxels 57.3 -> 22.4 ms; views
+// voxels, BF16 ring, 16.9 -> 5.9 ms (1360 G updates/s); FP32 ring, whose tile footprints
+// there did not fit a stage, 52.5 -> 6.2 ms; 400 x 400 x 317 voxels 57.3 -> 22.4 ms; views
 // that are not aligned with j, 16.9 -> 8.1 ms. What bounds it: four shared-memory loads a
 // sample (8 samples a clock and SM at most, 2270 G/s) beside 13 issue slots. Two CTAs an SM
 // with all the registers they want measured 6.5 ms.
@@ -29,14 +29,25 @@ namespace mr {
 constexpr int VB = 16;                            // block edge (voxels)
 constexpr int VB_CONSUMERS = 8;                   // consumer warps: one thread per (i, k) column
 constexpr int VB_THREADS = 32 * (VB_CONSUMERS + 1);
-constexpr int VB_CLUSTER = 4;                     // CTAs per block, each a quarter of the views
-constexpr int VB_MAXB = 8;                        // boxes of 8 rows per stage
 constexpr int VB_PAD = VB + 1;                    // partial sums: padded column of 16
 
 // Row pitches as in the staged kernel (bp_tma.cu); a 16-voxel block is half as tall, so a
-// stage holds 64 rows of either type and three CTAs fit an SM.
-template <typename T> struct BlockGeom { static constexpr int W = 88, ALIGN = 8, STAGES = 4; };
-template <> struct BlockGeom<float> { static constexpr int W = 84, ALIGN = 4, STAGES = 3; };
+// stage holds MAXB boxes of 8 rows, 64 of either type, and CTAS = three CTAs fit an SM.
+// COARSE: stages for blocks of voxels several detector pixels wide, whose footprints the plain
+// ones (76 x 60 pixels) do not hold: 124 columns by 124 rows, by 92 of an FP32 ring. Two of them,
+// so that three CTAs fit an SM (two of FP32). 600 views of 486 x 384, BF16, plain / coarse: 64 x
+// 64 x 51 voxels (7.6 pixels) 1.11 / 0.99 ms, 96 x 96 x 76 1.97 / 0.66, 128 x 128 x 102 (3.8
+// pixels) 2.86 / 1.11, 144 x 144 x 114 2.03 / 1.50; FP32 96 x 96 x 76 1.96 / 1.00, 128 x 128 x
+// 102 3.24 / 1.40 ms. 96 rows of BF16: 96 x 96 x 76 0.88 ms; 168 columns by 96 rows: 0.90 ms there,
+// 1.07 ms at 128 x 128 x 102; three stages, two CTAs: 0.84 and 1.15 ms.
+template <typename T, bool COARSE> struct BlockGeom {
+    static constexpr int W = 88, ALIGN = 8, STAGES = 4, MAXB = 8, CTAS = 3;
+};
+template <> struct BlockGeom<float, false> { static constexpr int W = 84, ALIGN = 4, STAGES = 3, MAXB = 8, CTAS = 3; };
+template <typename T> struct BlockGeom<T, true> {
+    static constexpr int W = 136, ALIGN = 8, STAGES = 2, MAXB = 16, CTAS = 3;
+};
+template <> struct BlockGeom<float, true> { static constexpr int W = 132, ALIGN = 4, STAGES = 2, MAXB = 12, CTAS = 2; };
 
 enum : int { VB_COLUMN = 3 };                     // beside MODE_STAGED / MODE_GLOBAL / MODE_SKIP
 
@@ -52,10 +63,11 @@ struct __align__(16) BlockMeta {
     int x0, r0, nbox, mode;
 };
 
-template <int KIND, typename T>
+template <int KIND, typename T, bool COARSE>
 __device__ __forceinline__ BlockMeta block_meta(const mr_view& V, const mr_grid& g, int i0, int j0, int k0, int R,
                                                 int C) {
-    constexpr int W = BlockGeom<T>::W, ALIGN = BlockGeom<T>::ALIGN;
+    using Geom = BlockGeom<T, COARSE>;
+    constexpr int W = Geom::W, ALIGN = Geom::ALIGN, MAXB = Geom::MAXB;
     float pu[4], pv[4];
     view_map(V, g, R, C, pu, pv);
     // the value at the block's origin in FP64: its FP32 rounding (half an ulp of a detector
@@ -109,12 +121,12 @@ __device__ __forceinline__ BlockMeta block_meta(const mr_view& V, const mr_grid&
     if (!behind && cmax == cmax && rmax == rmax && cmin == cmin && rmin == rmin) {
         if (cmax < -2.f || cmin > (float)C + 1.f || rmax < -2.f || rmin > (float)R + 1.f) {
             mode = MODE_SKIP;
-        } else if (cmax - cmin < (float)(W - ALIGN - 4) && rmax - rmin < (float)(ST_BOX_H * VB_MAXB - 4)) {
+        } else if (cmax - cmin < (float)(W - ALIGN - 4) && rmax - rmin < (float)(ST_BOX_H * MAXB - 4)) {
             x0 = ((int)floorf(cmin) - 1) & ~(ALIGN - 1);
             r0 = (int)floorf(rmin) - 1;
             const int rows = (int)floorf(rmax) + 3 - r0;
             nbox = (rows + ST_BOX_H - 1) / ST_BOX_H;
-            if ((int)floorf(cmax) + 3 - x0 <= W && nbox <= VB_MAXB)
+            if ((int)floorf(cmax) + 3 - x0 <= W && nbox <= MAXB)
                 mode = (au.w == 0.f && aw.w == 0.f) ? VB_COLUMN : MODE_STAGED;
         } else if (cmax - cmin < (float)(C + 2) && rmax - rmin < (float)(R + 2)) {
             // too wide to stage, on or near the detector: coordinates still count from a
@@ -161,20 +173,21 @@ __device__ __forceinline__ float2 lerp_pair(uint32_t a0, uint32_t a1, float2 fc,
 
 // Warp roles and the stage ring are those of bp_staged_kernel: warp 8 computes footprints
 // and issues the box loads, warps 0..7 sum; full / empty mbarriers with bounded waits. A
-// cluster of VB_CLUSTER CTAs splits the views of a block and adds the partial sums in rank
-// order through distributed shared memory, each rank finishing a quarter of the columns.
-template <int KIND, typename T>
-__global__ void __launch_bounds__(VB_THREADS, 3)
+// cluster of four or two CTAs (view_shares) splits the views of a block and adds the partial sums in rank
+// order through distributed shared memory, each rank finishing its share of the columns.
+template <int KIND, typename T, bool COARSE>
+__global__ void __launch_bounds__(VB_THREADS, BlockGeom<T, COARSE>::CTAS)
 bp_volume_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__ ring, int R, int C, int pitch,
                  long long slot_stride, int n_slots, const mr_view* __restrict__ views,
                  const __grid_constant__ mr_grid g, int blocks_i, int blocks_k, int blocks_j,
                  float* __restrict__ out, int* status) {
-    constexpr int W = BlockGeom<T>::W;
-    constexpr int S = BlockGeom<T>::STAGES;
+    using Geom = BlockGeom<T, COARSE>;
+    constexpr int W = Geom::W;
+    constexpr int S = Geom::STAGES;
     constexpr int ESZ = (int)sizeof(T);
     constexpr int PITCH = W * ESZ;
     constexpr int BOX_BYTES = PITCH * ST_BOX_H;
-    constexpr int STAGE_BYTES = BOX_BYTES * VB_MAXB;
+    constexpr int STAGE_BYTES = BOX_BYTES * Geom::MAXB;
     static_assert(BOX_BYTES % 128 == 0 && STAGE_BYTES % 128 == 0, "TMA box / stage not 128-byte aligned");
     static_assert(S * STAGE_BYTES >= VB_CONSUMERS * 32 * VB_PAD * 4, "partial sums reuse the stages");
 
@@ -218,7 +231,7 @@ bp_volume_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__
         for (int vb = 0; vb < nv; vb += 32) {
             const int cnt = min(32, nv - vb);
             __syncwarp();
-            if (lane < cnt) meta_new[lane] = block_meta<KIND, T>(views[v_begin + vb + lane], g, i0, j0, k0, R, C);
+            if (lane < cnt) meta_new[lane] = block_meta<KIND, T, COARSE>(views[v_begin + vb + lane], g, i0, j0, k0, R, C);
             __syncwarp();
             for (int l = 0; l < cnt; ++l) {
                 const uint32_t ua = (uint32_t)(vb + l);
@@ -355,27 +368,41 @@ bp_volume_kernel(const __grid_constant__ CUtensorMap tmap, const T* __restrict__
     cluster.sync();                             // partial sums stay alive until every rank has read them
 }
 
-template <int KIND, typename T>
+// CTAs per block, each a share of the views: four where two would leave SMs idle (below two and
+// a half blocks an SM), else two, which end and wait for one another half as often (600 views of
+// 486 x 384, BF16, four / two: 100 blocks 1.06 / 2.01 ms, 294 blocks 2.54 / 3.06, 384 blocks
+// 3.09 / 2.88, 800 blocks 1.70 / 1.64, 3328 blocks 6.19 / 5.88 ms).
+static unsigned view_shares(long long blocks) {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 148;
+    return 2 * blocks >= 5LL * sms ? 2u : 4u;
+}
+
+template <int KIND, bool COARSE, typename T>
 static int launch_volume(const mr_ring* ring, const mr_view* views, const mr_grid& g, float* out, int* status,
                          cudaStream_t st) {
     const long long bi = (g.n_i + VB - 1) / VB, bj = (g.n_j + VB - 1) / VB, bk = (g.n_k + VB - 1) / VB;
-    if (bi * bj > 2147483647LL / VB_CLUSTER || bi * bj * bk > 2147483647LL / VB_CLUSTER) return MR_ERR_UNSUPPORTED;
+    if (bi * bj > 2147483647LL / 4 || bi * bj * bk > 2147483647LL / 4) return MR_ERR_UNSUPPORTED;
+    const unsigned cluster = view_shares(bi * bj * bk);
+    using Geom = BlockGeom<T, COARSE>;
     CUtensorMap map;
-    int rc = make_ring_map<T>(ring, BlockGeom<T>::W, &map);
+    int rc = make_ring_map<T>(ring, Geom::W, &map);
     if (rc != MR_OK) return rc;
-    constexpr int S = BlockGeom<T>::STAGES;
-    const size_t smem = (size_t)S * BlockGeom<T>::W * ST_BOX_H * VB_MAXB * sizeof(T) + S * sizeof(BlockRec) +
+    constexpr int S = Geom::STAGES;
+    const size_t smem = (size_t)S * Geom::W * ST_BOX_H * Geom::MAXB * sizeof(T) + S * sizeof(BlockRec) +
                         32 * sizeof(BlockMeta) + 2 * S * sizeof(uint64_t) + 128;
-    auto kern = bp_volume_kernel<KIND, T>;
+    auto kern = bp_volume_kernel<KIND, T, COARSE>;
     MR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(bi * bj * bk * VB_CLUSTER));
+    cfg.gridDim = dim3((unsigned)(bi * bj * bk) * cluster);
     cfg.blockDim = dim3(VB_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = VB_CLUSTER;
+    attr[0].val.clusterDim.x = cluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
@@ -387,11 +414,10 @@ static int launch_volume(const mr_ring* ring, const mr_view* views, const mr_gri
     return MR_OK;
 }
 
-}  // namespace mr
-
-extern "C" int mr_backproject_volume(const mr_ring* ring, const mr_view* views, const mr_grid* grid, float* out,
-                                     int32_t* status, void* stream) {
-    int rc = mr::check_staged_ring(ring);
+template <bool COARSE>
+static int dispatch_volume(const mr_ring* ring, const mr_view* views, const mr_grid* grid, float* out, int32_t* status,
+                           void* stream) {
+    int rc = check_staged_ring(ring);
     if (rc != MR_OK) return rc;
     if (!views || !grid || !out || grid->n_i < 0 || grid->n_j < 0 || grid->n_k < 0) return MR_ERR_INVALID;
     if (grid->flags & (MR_GRID_POINTS | MR_GRID_MASK_BOX)) return MR_ERR_INVALID;
@@ -400,13 +426,25 @@ extern "C" int mr_backproject_volume(const mr_ring* ring, const mr_view* views, 
     const bool cone = ring->kind == MR_CONE;
     switch (ring->dtype) {
         case MR_F32:
-            return cone ? mr::launch_volume<MR_CONE, float>(ring, views, *grid, out, status, st)
-                        : mr::launch_volume<MR_PARALLEL, float>(ring, views, *grid, out, status, st);
+            return cone ? launch_volume<MR_CONE, COARSE, float>(ring, views, *grid, out, status, st)
+                        : launch_volume<MR_PARALLEL, COARSE, float>(ring, views, *grid, out, status, st);
         case MR_BF16:
-            return cone ? mr::launch_volume<MR_CONE, __nv_bfloat16>(ring, views, *grid, out, status, st)
-                        : mr::launch_volume<MR_PARALLEL, __nv_bfloat16>(ring, views, *grid, out, status, st);
+            return cone ? launch_volume<MR_CONE, COARSE, __nv_bfloat16>(ring, views, *grid, out, status, st)
+                        : launch_volume<MR_PARALLEL, COARSE, __nv_bfloat16>(ring, views, *grid, out, status, st);
         default:
-            return cone ? mr::launch_volume<MR_CONE, __half>(ring, views, *grid, out, status, st)
-                        : mr::launch_volume<MR_PARALLEL, __half>(ring, views, *grid, out, status, st);
+            return cone ? launch_volume<MR_CONE, COARSE, __half>(ring, views, *grid, out, status, st)
+                        : launch_volume<MR_PARALLEL, COARSE, __half>(ring, views, *grid, out, status, st);
     }
+}
+
+}  // namespace mr
+
+extern "C" int mr_backproject_volume(const mr_ring* ring, const mr_view* views, const mr_grid* grid, float* out,
+                                     int32_t* status, void* stream) {
+    return mr::dispatch_volume<false>(ring, views, grid, out, status, stream);
+}
+
+extern "C" int mr_backproject_volume_coarse(const mr_ring* ring, const mr_view* views, const mr_grid* grid, float* out,
+                                            int32_t* status, void* stream) {
+    return mr::dispatch_volume<true>(ring, views, grid, out, status, stream);
 }

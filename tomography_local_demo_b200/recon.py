@@ -245,6 +245,15 @@ RAW_LINE_BOUND = 11.1
 # four CTAs, so fewer than 64 leave SMs idle.
 BLOCK_VOLUME_MIN = 64
 
+# Voxel sizes, in detector pixels at the axis, of volumes that go to mr_backproject_volume_coarse.
+# Below, nearly every block's footprint fits a plain stage, of which more are in flight (3.2
+# pixels, 152 x 152 x 121 voxels of 600 cone views 1.82 ms, coarse 1.76; 80^3 of 180 parallel
+# views 0.116 and 0.126; 3.0 pixels, cone, 1.64 and 1.72; 3.4 pixels 2.03 and 1.50). Above, few fit
+# a coarse stage either, and the plain kernel's smaller ones leave more of L1 to the global loads
+# (7.6 pixels, 256 x 256 x 203 voxels of 120 full-resolution views 5.46 and 5.07 ms; 30 pixels,
+# 64 x 64 x 51 voxels 0.33 and 0.90).
+COARSE_VOXEL_PIXELS = (3.3, 8.0)
+
 # Width of a tile's side (31 sample steps) in detector pixels from which a grid goes to
 # mr_backproject_staged_wide. A view sees a square tile 1 to 1.4 sides wide and a stage takes 76
 # pixels, so from about 64 most views exceed it (25 axial 192^2 slices, side 81: 1739 -> 1003 us);
@@ -507,15 +516,24 @@ def is_block_volume(grids):
     return blocks >= BLOCK_VOLUME_MIN and 2 * math.prod(n) >= 4096 * blocks
 
 
-def backproject_volume_device(ring, views_dev, grid, out, stream, timer=None, status=None):
+def is_coarse_volume(grid, pixel):
+    """Whether a block volume goes to mr_backproject_volume_coarse: its largest step in detector
+    pixels at the axis (pixel: their size there) lies in COARSE_VOXEL_PIXELS."""
+    lo, hi = COARSE_VOXEL_PIXELS
+    step = max(math.sqrt(sum(x * x for x in grid[k].tolist())) for k in ("step_i", "step_j", "step_k"))
+    return lo * pixel < step < hi * pixel
+
+
+def backproject_volume_device(ring, views_dev, grid, out, stream, timer=None, status=None, coarse=False):
     """Back-project one regular grid (numpy GRID_DTYPE record, passed by value) in blocks
-    of 16^3 voxels into the device f32 tensor `out`."""
+    of 16^3 voxels into the device f32 tensor `out`. coarse: see is_coarse_volume."""
     v = ctypes_void
     rec = np.ascontiguousarray(grid, dtype=N.GRID_DTYPE).reshape(1)
     ev0 = timer.start(stream) if timer is not None else None
-    st = N.load().mr_backproject_volume(ring, v(views_dev.data_ptr()), rec.ctypes.data, v(out.data_ptr()),
-                                        v(status.data_ptr()) if status is not None else None,
-                                        v(stream.cuda_stream))
+    lib = N.load()
+    launch = lib.mr_backproject_volume_coarse if coarse else lib.mr_backproject_volume
+    st = launch(ring, v(views_dev.data_ptr()), rec.ctypes.data, v(out.data_ptr()),
+                v(status.data_ptr()) if status is not None else None, v(stream.cuda_stream))
     if timer is not None:
         timer.stop("mr_backproject_volume", ev0, stream)
     N.check(st, "mr_backproject_volume")
@@ -1287,12 +1305,13 @@ class SliceReconstructor:
         regular = not (np.asarray(grids["flags"]) & N.MR_GRID_POINTS).any()
         if self.bp_kernel == "staged" and is_block_volume(grids):
             bounds = [0] + [se for se, _ in marks] + [n]
+            coarse = is_coarse_volume(grids[0], self.native_pixel)
             for a, b, e in zip(bounds[:-1], bounds[1:], [e for _, e in marks] + [event]):
                 if e is not None:
                     stream.wait_event(e)
                 grids["view_begin"], grids["n_views"], grids["accumulate"] = a, b - a, int(a > 0)
                 backproject_volume_device(self._ring_c, self._views_dev, grids, out, stream, self.kernel_timer,
-                                          self._status)
+                                          self._status, coarse)
             return
         if marks and regular and self.bp_kernel == "staged":
             bounds = [0] + [se for se, _ in marks] + [n]
