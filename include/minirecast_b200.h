@@ -169,12 +169,29 @@ int mr_backproject_staged(const mr_ring* ring, const mr_view* views_dev,
                           const mr_grid* grids_dev, const mr_tile* tiles_dev, int64_t n_tiles,
                           float* out_dev, int32_t* status_dev, void* stream);
 
+/* The same, bit for bit, with half the warps a tile and more tiles at once: faster for launches of
+ * many tiles whose footprints are staged (at most 76 columns x 76 rows, 76 x 60 of an FP32 ring),
+ * slower for others. mr_staged_traits tells how a grid's are. */
+int mr_backproject_staged_slim(const mr_ring* ring, const mr_view* views_dev,
+                               const mr_grid* grids_dev, const mr_tile* tiles_dev, int64_t n_tiles,
+                               float* out_dev, int32_t* status_dev, void* stream);
+
 /* The same, bit for bit, for grids whose samples lie a few detector pixels apart: footprints of
  * a tile that are wide and flat (up to 252 columns x 16 rows or 168 x 32; 248 x 24 or 176 x 40
  * for 16-bit rings) are staged too, where mr_backproject_staged reads global memory. */
 int mr_backproject_staged_wide(const mr_ring* ring, const mr_view* views_dev,
                                const mr_grid* grids_dev, const mr_tile* tiles_dev, int64_t n_tiles,
                                float* out_dev, int32_t* status_dev, void* stream);
+
+/* What chooses between the three forms, on the host alone. mr_staged_traits looks at 64 (tile,
+ * view) pairs of one regular grid: traits = {tiles that may hold a sample inside the box, share
+ * of the pairs whose footprint mr_backproject_staged stages (or skips), share that only
+ * mr_backproject_staged_wide does}; views_host: the views' records; kind, rows, cols, dtype: the
+ * ring's. mr_staged_slim_pays: 1 when mr_backproject_staged_slim is the faster form for a launch
+ * of that many busy tiles, all of whose footprints are staged, else 0. */
+int mr_staged_traits(const mr_view* views_host, int32_t n_views, int32_t kind, int32_t rows,
+                     int32_t cols, int32_t dtype, const mr_grid* grid_host, double* traits);
+int mr_staged_slim_pays(int64_t busy_tiles, int32_t dtype);
 
 /* The same sum over one regular grid (no flags) that is deep along i, j and k: a volume,
  * in blocks of 16 x 16 x 16 voxels whose footprints are staged once per view. Views whose

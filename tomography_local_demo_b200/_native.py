@@ -63,6 +63,9 @@ SIGNATURES = {
     "mr_backproject": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P]),
     "mr_backproject_staged": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P, _P]),
     "mr_backproject_staged_wide": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P, _P]),
+    "mr_backproject_staged_slim": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _I64, _P, _P, _P]),
+    "mr_staged_traits": (ctypes.c_int, [_P, _I32, _I32, _I32, _I32, _I32, _P, _P]),
+    "mr_staged_slim_pays": (ctypes.c_int, [_I64, _I32]),
     "mr_backproject_volume": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _P]),
     "mr_backproject_volume_coarse": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _P]),
     "mr_backproject_persistent": (ctypes.c_int, [ctypes.POINTER(MrRing), _P, _P, _P, _P, _I64, _P, _P, _P, _P]),

@@ -91,18 +91,22 @@ __device__ __forceinline__ bool in_box_fp64_t(const mr_grid& g, int i, int j) {
     return ok;
 }
 
-// Per-view footprint + local affine coefficients of one tile (computed by one lane of
-// the producer warp).
+// Where one tile lies in a view, and how its footprint is read: the affine maps of column and
+// row numerator and depth, (value at the tile origin, d/di, d/dj), and the boxes.
+struct Footprint {
+    float3 au, av, aw;
+    int x0, r0, nbox, mode;
+};
 template <int KIND, bool WIDE, typename T>
-__device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g, float ox, float oy,
-                                              float oz, int di_max, int dj_max, int R, int C) {
+__host__ __device__ __forceinline__ Footprint footprint(const mr_view& V, const mr_grid& g, float ox, float oy,
+                                                        float oz, int di_max, int dj_max, int R, int C) {
     constexpr int W = StageGeom<T>::W;
     float pu[4], pv[4];
     view_map(V, g, R, C, pu, pv);
     auto aff = [&](const float* m) {
-        return make_float3(fmaf(m[0], ox, fmaf(m[1], oy, fmaf(m[2], oz, m[3]))),
-                           fmaf(m[0], g.step_i[0], fmaf(m[1], g.step_i[1], m[2] * g.step_i[2])),
-                           fmaf(m[0], g.step_j[0], fmaf(m[1], g.step_j[1], m[2] * g.step_j[2])));
+        return make_float3(mul_add(m[0], ox, mul_add(m[1], oy, mul_add(m[2], oz, m[3]))),
+                           mul_add(m[0], g.step_i[0], mul_add(m[1], g.step_i[1], m[2] * g.step_i[2])),
+                           mul_add(m[0], g.step_j[0], mul_add(m[1], g.step_j[1], m[2] * g.step_j[2])));
     };
     float3 au = aff(pu), av = aff(pv), aw = aff(V.pw);
     if (KIND == MR_CONE && V.qscale != 1.f) {
@@ -118,9 +122,9 @@ __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g
     for (int c = 0; c < 4; ++c) {
         const float di = (c & 1) ? (float)di_max : 0.f;
         const float dj = (c & 2) ? (float)dj_max : 0.f;
-        const float w = fmaf(di, aw.y, fmaf(dj, aw.z, aw.x));
-        float cc = fmaf(di, au.y, fmaf(dj, au.z, au.x));
-        float rr = fmaf(di, av.y, fmaf(dj, av.z, av.x));
+        const float w = mul_add(di, aw.y, mul_add(dj, aw.z, aw.x));
+        float cc = mul_add(di, au.y, mul_add(dj, au.z, au.x));
+        float rr = mul_add(di, av.y, mul_add(dj, av.z, av.x));
         if (KIND == MR_CONE) {
             behind |= !(w > 1e-3f);
             const float inv = 1.f / w;
@@ -130,7 +134,6 @@ __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g
         cmin = fminf(cmin, cc); cmax = fmaxf(cmax, cc);
         rmin = fminf(rmin, rr); rmax = fmaxf(rmax, rr);
     }
-    ViewMeta m;
     int mode = MODE_GLOBAL, x0 = 0, r0 = 0, nbox = 0;
     if (!behind && cmax == cmax && rmax == rmax && cmin == cmin && rmin == rmin) {
         if (cmax < -2.f || cmin > (float)C + 1.f || rmax < -2.f || rmin > (float)R + 1.f) {
@@ -152,6 +155,19 @@ __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g
             else if (wide <= StageGeom<T>::W3 && nbox <= StageGeom<T>::MAXB3) mode = MODE_WIDE3;
         }
     }
+    return Footprint{au, av, aw, x0, r0, nbox, mode};
+}
+
+// Per-view footprint + local affine coefficients of one tile (computed by one lane of
+// the producer warp).
+template <int KIND, bool WIDE, typename T>
+__device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g, float ox, float oy,
+                                              float oz, int di_max, int dj_max, int R, int C) {
+    constexpr int W = StageGeom<T>::W;
+    const Footprint f = footprint<KIND, WIDE, T>(V, g, ox, oy, oz, di_max, dj_max, R, C);
+    const float3 au = f.au, av = f.av, aw = f.aw;
+    const int x0 = f.x0, r0 = f.r0, nbox = f.nbox, mode = f.mode;
+    ViewMeta m;
     float3 cu = au, cv = av;
     if (mode == MODE_STAGED) {
         const float fx0 = (float)x0, fr0 = (float)r0;
@@ -571,23 +587,6 @@ static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_gri
     return MR_OK;
 }
 
-// Whether a launch of n tiles is faster with SLIM: its CTAs take 1.47 (FP32: 1.24) times as long,
-// but 5/3 (4/3) as many run at once. A launch of x waves costs between x and the next whole
-// number of them; half way between is taken (one slice, 600 views, BF16, full / slim: 64 tiles
-// 340 / 602 us, 144 tiles 196 / 150, 256 tiles 284 / 256, 300 tiles 323 / 305, 625 tiles 597 /
-// 540; FP32, 300 tiles 324 / 362, 256 tiles 283 / 265).
-static bool slim_pays(int64_t n, bool fp32) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        sms = 148;
-    auto cost = [&](int ctas, double time) {
-        const double x = (double)n * ST_CLUSTER / ((double)sms * ctas);
-        return 0.5 * (x + ceil(x)) * time;
-    };
-    return cost(fp32 ? 4 : 5, fp32 ? 1.24 : 1.47) < cost(3, 1.0);
-}
-
 template <bool WIDE, bool SLIM, typename... Args>
 static int dispatch_staged(const mr_ring* ring, Args... args) {
     const bool cone = ring->kind == MR_CONE;
@@ -604,35 +603,119 @@ static int dispatch_staged(const mr_ring* ring, Args... args) {
     }
 }
 
+// Whether a launch of n busy tiles whose footprints are staged is faster with SLIM: its CTAs take
+// 1.47 (FP32: 1.24) times as long, but 175 (142) clusters run at once where 104 of the full form do
+// (cudaOccupancyMaxActiveClusters, 148 SMs: fewer than the CTAs an SM would give, as a cluster
+// stays inside a GPC). A launch of x waves costs between x and the next whole number of them; half
+// way between is taken. Of 3076 random lists of slices (1 to 25 slices of 64 to 1024 samples a
+// side, 40 to 600 views, six detectors) it takes 889, none of them slower: 0.70 to 1.0 times the
+// full form's time, 0.86 in the median. By the CTAs an SM alone (111, 148 and 185 clusters), and
+// with tiles counted that lie outside the box or read global memory, 730 of 2024 were slower,
+// up to 2.0 times.
+static bool slim_pays(int64_t n, bool fp32) {
+    auto cost = [&](int clusters, double time) {
+        const double x = (double)n / clusters;
+        return 0.5 * (x + ceil(x)) * time;
+    };
+    return cost(fp32 ? 142 : 175, fp32 ? 1.24 : 1.47) < cost(104, 1.0);
+}
+
+// Tiles of a regular grid that may hold a sample inside the box (all of them without a mask):
+// those whose centre lies no further outside than the tile reaches.
+template <typename F>
+static int64_t for_busy_tiles(const mr_grid& g, F each) {
+    const bool mask = (g.flags & MR_GRID_MASK_BOX) != 0;
+    const double half = 0.5 * (ST_TI - 1) * fabs(g.mask_delta);
+    double reach[3];
+    for (int e = 0; e < 3; ++e) reach[e] = g.box[e] + half * (fabs(g.mask_ej[e]) + fabs(g.mask_ei[e])) * (1 + 1e-9);
+    int64_t n = 0;
+    for (int32_t k = 0; k < g.n_k; ++k)
+        for (int32_t i0 = 0; i0 < g.n_i; i0 += ST_TI)
+            for (int32_t j0 = 0; j0 < g.n_j; j0 += ST_TJ) {
+                const double ai = (i0 + 0.5 * (ST_TI - 1) - g.mask_half) * g.mask_delta;
+                const double aj = (j0 + 0.5 * (ST_TJ - 1) - g.mask_half) * g.mask_delta;
+                bool in = true;
+                for (int e = 0; mask && e < 3; ++e)
+                    in = in && fabs(g.mask_c[e] + aj * g.mask_ej[e] + ai * g.mask_ei[e]) <= reach[e];
+                if (in) each(n++, i0, j0, k);
+            }
+    return n;
+}
+
+constexpr int TRAIT_PAIRS = 64;                   // (tile, view) pairs looked at
+
+// How the footprints of TRAIT_PAIRS busy tiles, spread over the grid, are read, each in a view of
+// its own: count[0] from a stage (or not at all), count[1] from a wide box. The views run round
+// the orbit 27 times while the tiles run once through the grid.
+template <int KIND, typename T>
+static void pair_modes(const mr_view* views, int n_views, const mr_grid& g, int R, int C, int64_t busy, int* count) {
+    int64_t pair = 0;
+    for_busy_tiles(g, [&](int64_t at, int32_t i0, int32_t j0, int32_t k) {
+        for (; pair < TRAIT_PAIRS && pair * busy / TRAIT_PAIRS == at; ++pair) {
+            const mr_view& V = views[pair * 27 % TRAIT_PAIRS * n_views / TRAIT_PAIRS];
+            const float x = g.origin[0] + i0 * g.step_i[0] + j0 * g.step_j[0] + k * g.step_k[0];
+            const float y = g.origin[1] + i0 * g.step_i[1] + j0 * g.step_j[1] + k * g.step_k[1];
+            const float z = g.origin[2] + i0 * g.step_i[2] + j0 * g.step_j[2] + k * g.step_k[2];
+            const int di = g.n_i - i0 < ST_TI ? g.n_i - i0 - 1 : ST_TI - 1;
+            const int dj = g.n_j - j0 < ST_TJ ? g.n_j - j0 - 1 : ST_TJ - 1;
+            const int mode = footprint<KIND, true, T>(V, g, x, y, z, di, dj, R, C).mode;
+            count[0] += mode == MODE_STAGED || mode == MODE_SKIP;
+            count[1] += mode == MODE_WIDE2 || mode == MODE_WIDE3;
+        }
+    });
+}
+
 }  // namespace mr
 
-extern "C" int mr_backproject_staged(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
-                                     const mr_tile* tiles, int64_t n_tiles, float* out, int32_t* status,
-                                     void* stream) {
+extern "C" int mr_staged_traits(const mr_view* views, int32_t n_views, int32_t kind, int32_t rows, int32_t cols,
+                                int32_t dtype, const mr_grid* grid, double* traits) {
+    if (!views || n_views < 1 || !grid || !traits || rows < 1 || cols < 1) return MR_ERR_INVALID;
+    if (grid->n_i < 0 || grid->n_j < 0 || grid->n_k < 0 || (grid->flags & MR_GRID_POINTS)) return MR_ERR_INVALID;
+    if (kind != MR_CONE && kind != MR_PARALLEL) return MR_ERR_INVALID;
+    if (dtype != MR_F32 && dtype != MR_BF16 && dtype != MR_F16) return MR_ERR_INVALID;
+    const int64_t busy = mr::for_busy_tiles(*grid, [](int64_t, int32_t, int32_t, int32_t) {});
+    int count[2] = {0, 0};
+    auto modes = dtype == MR_F32 ? (kind == MR_CONE ? mr::pair_modes<MR_CONE, float> : mr::pair_modes<MR_PARALLEL, float>)
+                                 : (kind == MR_CONE ? mr::pair_modes<MR_CONE, __half> : mr::pair_modes<MR_PARALLEL, __half>);
+    if (busy > 0) modes(views, n_views, *grid, rows, cols, busy, count);    // both 16-bit types have the same stages
+    traits[0] = (double)busy;
+    traits[1] = busy > 0 ? (double)count[0] / mr::TRAIT_PAIRS : 1.0;
+    traits[2] = (double)count[1] / mr::TRAIT_PAIRS;
+    return MR_OK;
+}
+
+extern "C" int mr_staged_slim_pays(int64_t busy_tiles, int32_t dtype) {
+    return mr::slim_pays(busy_tiles, dtype == MR_F32) ? 1 : 0;
+}
+
+template <bool WIDE, bool SLIM>
+static int backproject_staged(const mr_ring* ring, const mr_view* views, const mr_grid* grids, const mr_tile* tiles,
+                              int64_t n_tiles, float* out, int32_t* status, void* stream) {
     int rc = mr::check_staged_ring(ring);
     if (rc != MR_OK) return rc;
     if (!views || !grids || !out || n_tiles < 0 || (n_tiles > 0 && !tiles)) return MR_ERR_INVALID;
     if (n_tiles == 0) return MR_OK;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int64_t* no_count = nullptr;
-    unsigned int* no_counter = nullptr;
-    return mr::slim_pays(n_tiles, ring->dtype == MR_F32)
-               ? mr::dispatch_staged<false, true>(ring, views, grids, tiles, n_tiles, out, status, st, no_count,
-                                                  no_counter)
-               : mr::dispatch_staged<false, false>(ring, views, grids, tiles, n_tiles, out, status, st, no_count,
-                                                   no_counter);
+    return mr::dispatch_staged<WIDE, SLIM>(ring, views, grids, tiles, n_tiles, out, status,
+                                           static_cast<cudaStream_t>(stream), (const int64_t*)nullptr,
+                                           (unsigned int*)nullptr);
+}
+
+extern "C" int mr_backproject_staged(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
+                                     const mr_tile* tiles, int64_t n_tiles, float* out, int32_t* status,
+                                     void* stream) {
+    return backproject_staged<false, false>(ring, views, grids, tiles, n_tiles, out, status, stream);
+}
+
+extern "C" int mr_backproject_staged_slim(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
+                                          const mr_tile* tiles, int64_t n_tiles, float* out, int32_t* status,
+                                          void* stream) {
+    return backproject_staged<false, true>(ring, views, grids, tiles, n_tiles, out, status, stream);
 }
 
 extern "C" int mr_backproject_staged_wide(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
                                           const mr_tile* tiles, int64_t n_tiles, float* out, int32_t* status,
                                           void* stream) {
-    int rc = mr::check_staged_ring(ring);
-    if (rc != MR_OK) return rc;
-    if (!views || !grids || !out || n_tiles < 0 || (n_tiles > 0 && !tiles)) return MR_ERR_INVALID;
-    if (n_tiles == 0) return MR_OK;
-    return mr::dispatch_staged<true, false>(ring, views, grids, tiles, n_tiles, out, status,
-                                     static_cast<cudaStream_t>(stream), (const int64_t*)nullptr,
-                                     (unsigned int*)nullptr);
+    return backproject_staged<true, false>(ring, views, grids, tiles, n_tiles, out, status, stream);
 }
 
 extern "C" int mr_backproject_persistent(const mr_ring* ring, const mr_view* views, const mr_grid* grids,

@@ -63,17 +63,27 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 
+// a b + c, for code that the host also runs to see what a kernel will do: one rounding on the
+// device; two on the host, whose fmaf is a library call of some 20 ns where no FMA is assumed.
+__host__ __device__ __forceinline__ float mul_add(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+    return fmaf(a, b, c);
+#else
+    return a * b + c;
+#endif
+}
+
 // Per-view projective map with the grid's COR shift and detector tilt applied:
 //   no tilt: pu' = pu + shift pw,  pv' = pv + shift uv pw                 (recon.py:420)
 //   tilt   : (col, row) rotated by the tilt about the detector centre, then shifted.
-__device__ __forceinline__ void view_map(const mr_view& V, const mr_grid& g, int R, int C, float* pu,
+__host__ __device__ __forceinline__ void view_map(const mr_view& V, const mr_grid& g, int R, int C, float* pu,
                                          float* pv) {
     const float shift = g.cor_shift;
     if (g.tilt_cos == 0.f && g.tilt_sin == 0.f) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            pu[e] = fmaf(shift, V.pw[e], V.pu[e]);
-            pv[e] = fmaf(shift * V.uv, V.pw[e], V.pv[e]);
+            pu[e] = mul_add(shift, V.pw[e], V.pu[e]);
+            pv[e] = mul_add(shift * V.uv, V.pw[e], V.pv[e]);
         }
     } else {
         const float c = g.tilt_cos, s = g.tilt_sin;
@@ -82,8 +92,8 @@ __device__ __forceinline__ void view_map(const mr_view& V, const mr_grid& g, int
         const float kv = cr * (1.f - c) + cc * s + shift * V.uv;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            pu[e] = fmaf(c, V.pu[e], fmaf(s, V.pv[e], ku * V.pw[e]));
-            pv[e] = fmaf(-s, V.pu[e], fmaf(c, V.pv[e], kv * V.pw[e]));
+            pu[e] = mul_add(c, V.pu[e], mul_add(s, V.pv[e], ku * V.pw[e]));
+            pv[e] = mul_add(-s, V.pu[e], mul_add(c, V.pv[e], kv * V.pw[e]));
         }
     }
 }

@@ -261,6 +261,13 @@ COARSE_VOXEL_PIXELS = (3.3, 8.0)
 # 1316 us with the wide variant).
 WIDE_TILE_PIXELS = 64
 
+# Share of a grid's (tile, view) pairs whose footprint a stage holds, from which the grid may go
+# to mr_backproject_staged_slim. Its four warps hide less of the latency of footprints read from
+# global memory: lists whose grids all have 0.97 or more took 0.70 to 1.0 times the full form's
+# time, from 0.95 on up to 1.1, without the condition up to 1.7 (the 3076 lists described at the
+# count of tiles that pays, mr_staged_slim_pays).
+SLIM_SHARE = 0.97
+
 
 def _device(device=None):
     if not torch.cuda.is_available():
@@ -432,7 +439,7 @@ class KernelTimer:
 
 
 def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, kernel="staged",
-                       status=None, wait=None, asynchronous=False, band_axis=None, wide=None):
+                       status=None, wait=None, asynchronous=False, band_axis=None, wide=None, slim=False):
     """Back-project numpy GRID_DTYPE records into the device f32 tensor `out`.
 
     kernel="staged": regular grids go through mr_backproject_staged (TMA-staged
@@ -443,7 +450,8 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     page-locked memory with asynchronous=True). band_axis: the orbit's rotation axis, which
     orders the tiles of regular grids by height (_native.plan_tiles). wide: which grids go
     through mr_backproject_staged_wide (the same result bit for bit; see is_wide), one truth
-    value each, or None for none."""
+    value each, or None for none. slim: whether the others go through
+    mr_backproject_staged_slim (the same result bit for bit; see slim_pays)."""
     grids = np.ascontiguousarray(grids, dtype=N.GRID_DTYPE)
     is_pts = (grids["flags"] & N.MR_GRID_POINTS) != 0
     if kernel == "staged" and is_pts.any() and not is_pts.all():
@@ -457,7 +465,7 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
         w = np.asarray(wide, dtype=bool)
         for part, flag in ((grids[w], [True] * int(w.sum())), (grids[~w], None)):
             backproject_device(ring, views_dev, part, out, stream, device, timer, kernel, status, wait, asynchronous,
-                               band_axis, flag)
+                               band_axis, flag, slim)
             wait = None
         return
     tiles = N.plan_tiles(grids, band_axis)
@@ -477,7 +485,7 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     name = "mr_backproject_staged" if staged else "mr_backproject"
     ev0 = timer.start(stream) if timer is not None else None
     if staged:
-        fn = lib.mr_backproject_staged_wide if all_wide else lib.mr_backproject_staged
+        fn = staged_entry(lib, all_wide, slim)
         st = fn(ring, v(views_dev.data_ptr()), v(g_ptr), v(t_ptr), len(tiles), v(out.data_ptr()),
                 v(status.data_ptr()) if status is not None else None, v(stream.cuda_stream))
     else:
@@ -488,6 +496,28 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     N.check(st, name)
     # keep the descriptor tensor alive until the kernel has consumed it
     recs.record_stream(stream)
+
+
+def staged_entry(lib, wide, slim):
+    """The library's entry of that form of the staged back-projection."""
+    if wide:
+        return lib.mr_backproject_staged_wide
+    return lib.mr_backproject_staged_slim if slim else lib.mr_backproject_staged
+
+
+def staged_traits(maps, kind_code, rows, cols, dtype_code, grid):
+    """mr_staged_traits of one regular grid (a record's bytes) over the views `maps` (numpy
+    VIEW_DTYPE records): (busy tiles, share of staged footprints, share that only wide boxes hold)."""
+    t = (ctypes.c_double * 3)()
+    N.check(N.load().mr_staged_traits(maps.ctypes.data, len(maps), kind_code, rows, cols, dtype_code, grid, t),
+            "mr_staged_traits")
+    return int(t[0]), t[1], t[2]
+
+
+def slim_pays(traits, dtype_code):
+    """Whether grids of these traits, in one launch, go to mr_backproject_staged_slim."""
+    return (all(share >= SLIM_SHARE for _, share, _ in traits)
+            and bool(N.load().mr_staged_slim_pays(sum(t[0] for t in traits), dtype_code)))
 
 
 def is_wide(grid, band_axis, wide_step):
@@ -1293,12 +1323,13 @@ class SliceReconstructor:
         with self._lock:
             return self.n, self.cor_shift, self._ingest_event
 
-    def _run_grids(self, grids, out, n, event, wide=None):
+    def _run_grids(self, grids, out, n, event, wide=None, slim=None):
         """Launch the batched back-projection of `grids` into device `out`. Right after a
         chunked host upload, the views are summed chunk by chunk: each partial launch
         waits only for its own chunk's filter, so the reconstruction overlaps the transfer
         of the later chunks (same scale; FP32 partial sums added in view order). Called with the
-        device and the reconstruction stream current. wide: see backproject_device."""
+        device and the reconstruction stream current. wide, slim: see backproject_device (slim
+        None: found out here)."""
         stream = self.stream
         grids["scale"] = np.pi / n if n else 0.0
         marks = [(se, e) for se, e in self._chunk_marks if 0 < se < n]
@@ -1313,6 +1344,8 @@ class SliceReconstructor:
                 backproject_volume_device(self._ring_c, self._views_dev, grids, out, stream, self.kernel_timer,
                                           self._status, coarse)
             return
+        if slim is None and regular and self.bp_kernel == "staged":
+            slim = slim_pays([self._traits(g.tobytes()) for g in grids], self._dtype_code)
         if marks and regular and self.bp_kernel == "staged":
             bounds = [0] + [se for se, _ in marks] + [n]
             events = [e for _, e in marks] + [event]
@@ -1326,7 +1359,7 @@ class SliceReconstructor:
             if len(tiles) == 0:
                 return
             lib = N.load()
-            launch = lib.mr_backproject_staged_wide if wide and all(wide) else lib.mr_backproject_staged
+            launch = staged_entry(lib, wide and all(wide), slim and not (wide and any(wide)))
             v = ctypes_void
             with torch.cuda.device(self.device), torch.cuda.stream(stream):
                 # one upload for all ranges and the tiles; launch i reads its own G records
@@ -1351,7 +1384,8 @@ class SliceReconstructor:
         # the copy engines): the records go up without the host waiting
         backproject_device(self._ring_c, self._views_dev, grids, out, stream, self.device,
                            self.kernel_timer, self.bp_kernel, self._status, wait=event,
-                           asynchronous=not self._chunk_marks, band_axis=self._band_axis, wide=wide)
+                           asynchronous=not self._chunk_marks, band_axis=self._band_axis, wide=wide,
+                           slim=bool(slim))
 
     def reconstruct_points_tensor(self, pts, cor_shift=None):
         """Device variant of reconstruct_points: pts (M, 3) -> f32 tensor [M]."""
@@ -1384,10 +1418,14 @@ class SliceReconstructor:
         shift = self.cor_shift if cor_shift is None else float(cor_shift)
         return plane_grid(self.box, origin, normal, int(n), size, zoom, center, shift)
 
+    def _traits(self, grid):
+        """staged_traits of a grid record's bytes over the orbit's views."""
+        return staged_traits(self._maps_all, self._kind_code, self.geom.rows, self.geom.cols, self._dtype_code, grid)
+
     def _plane_entry(self, origin, normal, n, size, zoom, center, shift):
-        """(record bytes, wide) of plane_grid for this reconstructor's box, memoised on the
+        """(record bytes, wide, traits) of plane_grid for this reconstructor's box, memoised on the
         request's parameters (the FP64 plane set-up is pure; a repeated request skips it on the
-        host). wide: see is_wide."""
+        host). wide: see is_wide; traits: see staged_traits."""
         scale = (n, None if size is None else float(size), float(zoom), float(shift))
         try:
             key = (tuple(map(float, origin)), tuple(map(float, normal)),
@@ -1399,7 +1437,8 @@ class SliceReconstructor:
         entry = cache.get(key)
         if entry is None:
             rec = plane_grid(self.box, origin, normal, n, size, zoom, center, shift)
-            entry = (rec.tobytes(), is_wide(rec, self._band_axis, self._wide_step))
+            raw = rec.tobytes()
+            entry = (raw, is_wide(rec, self._band_axis, self._wide_step), self._traits(raw))
             cache[key] = entry
             if len(cache) > 256:
                 cache.popitem(last=False)
@@ -1407,10 +1446,10 @@ class SliceReconstructor:
             cache.move_to_end(key)
         return entry
 
-    def _plane_record(self, origin, normal, n, size, zoom, center, shift):
-        """The mr_grid record of _plane_entry."""
-        rec = self._plane_entry(origin, normal, int(n), size, zoom, center, shift)[0]
-        return np.frombuffer(bytearray(rec), dtype=N.GRID_DTYPE)[0]
+    def _forms(self, entries):
+        """(wide, slim) of backproject_device for a list of _plane_entry's."""
+        wide = [e[1] for e in entries]
+        return wide, slim_pays([e[2] for e in entries if not e[1]], self._dtype_code)
 
     def _planes(self, requests):
         """One batched launch for many slices -> (flat f32 device tensor, sizes)."""
@@ -1431,7 +1470,7 @@ class SliceReconstructor:
             if n_views > 0 and offset > 0:
                 # every sample of every grid is written, those outside the box as 0
                 out = torch.empty(offset, dtype=torch.float32, device=self.device)
-                self._run_grids(grids, out, n_views, ev, [e[1] for e in entries])
+                self._run_grids(grids, out, n_views, ev, *self._forms(entries))
             else:
                 out = torch.zeros(offset, dtype=torch.float32, device=self.device)
         _handoff(self.stream, out)
@@ -1751,18 +1790,20 @@ class ScanReplay:
         dev = rec.device
         # records, bound for the whole life of the graph
         fv_host = rec._filter_views(self.indices, self.indices)
-        grids = np.zeros(len(requests), dtype=N.GRID_DTYPE)
-        sizes, offset = [], 0
-        for r, req in enumerate(requests):
+        entries, sizes, offsets, offset = [], [], [], 0
+        for req in requests:
             n = int(req.get("n", 256))
             s_ = req.get("cor_shift")
-            grids[r] = rec._plane_record(req["origin"], req["normal"], n, req.get("size"), req.get("zoom", 1.0),
-                                         req.get("center"), rec.cor_shift if s_ is None else float(s_))
-            grids[r]["out_offset"] = offset
+            entries.append(rec._plane_entry(req["origin"], req["normal"], n, req.get("size"), req.get("zoom", 1.0),
+                                            req.get("center"), rec.cor_shift if s_ is None else float(s_)))
+            offsets.append(offset)
             sizes.append(n)
             offset += n * n
+        grids = np.frombuffer(bytearray(b"".join([e[0] for e in entries])), dtype=N.GRID_DTYPE)
+        grids["out_offset"] = offsets
         grids["n_views"] = k
         grids["scale"] = np.pi / k
+        self._slim = slim_pays([e[2] for e in entries], rec._dtype_code)
         tiles = N.plan_tiles(grids, rec._band_axis)
         self.stream = torch.cuda.Stream(dev)
         rec.reset()
@@ -1806,7 +1847,7 @@ class ScanReplay:
             return
         lib, v = N.load(), ctypes_void
         base = self.recs.data_ptr()
-        fn = lib.mr_backproject_staged if rec.bp_kernel == "staged" else lib.mr_backproject
+        fn = staged_entry(lib, False, self._slim) if rec.bp_kernel == "staged" else lib.mr_backproject
         name = "mr_backproject_staged" if rec.bp_kernel == "staged" else "mr_backproject"
         args = [rec._ring_c, v(rec._views_dev.data_ptr()), v(base + self._g_off), v(base + self._t_off),
                 self.n_tiles, v(self.out.data_ptr())]
