@@ -67,6 +67,23 @@ def test_launches_of_the_four_warp_form():
         assert not R.slim_pays([], dtype)
 
 
+@pytest.mark.parametrize("dtype", [N.MR_F32, N.MR_BF16])
+def test_only_footprints_that_wide_boxes_hold_are_wide(dtype):
+    def chosen(normal, pixels, count, n=192):
+        grids = [R.plane_grid(3 * GEOM.volume_box(), (0, 0, 0.5), normal, n, n * pixels * PIXEL)] * count
+        wide = [R.is_wide(g, (0.0, 0.0, 1.0), R.WIDE_TILE_PIXELS / 31 * PIXEL) for g in grids]
+        assert wide == [True] * count
+        return R.wide_grids(wide, [traits(g, dtype) for g in grids])
+    assert chosen((0, 0, 1.0), 2.6, 25) == [True] * 25           # trial slices of a rotation-centre search
+    assert chosen((0, 0, 1.0), 2.6, 1) == [True]
+    assert chosen((0, 1.0, 0), 3.0, 25) == [False] * 25          # as tall as wide
+    assert chosen((0.5, 0.4, 0.7), 3.0, 25) == [False] * 25
+    assert chosen((0, 0, 1.0), 14.0, 25, 64) == [False] * 25     # 434 columns
+    # 186 to 263 columns: a part of the views is in a box, which one slice's tiles do not wait for
+    assert chosen((0, 0, 1.0), 6.0, 25, 96) == [True] * 25
+    assert chosen((0, 0, 1.0), 6.0, 1, 96) == [False]
+
+
 def test_traits_argument_checks():
     lib, t = N.load(), (ctypes.c_double * 3)()
     ok = [MAPS.ctypes.data, VIEWS, N.MR_CONE, ROWS, COLS, N.MR_F32, plane((0, 0, 1.0), 64).tobytes(), t]
@@ -76,3 +93,18 @@ def test_traits_argument_checks():
     points = plane((0, 0, 1.0), 64)
     points["flags"] = N.MR_GRID_POINTS
     assert lib.mr_staged_traits(*(ok[:6] + [points.tobytes(), t])) == N.MR_ERR_INVALID
+
+
+@pytest.mark.parametrize("dtype", [N.MR_F32, N.MR_BF16, N.MR_F16])
+def test_both_wide_boxes_occur_where_they_are_compared(dtype):
+    """The geometry of test_wide_boxes_change_nothing: tilted slices whose footprints are too tall
+    for FP32's wider box, axial ones that are too wide for the narrower box."""
+    from oracle import geometry as og
+    maps = R.cone_view_maps(R.cone_constants(og.circular_cone_vectors(29, 440.0, 680.0, 0.3)), 90, 420)
+    pixel, box = 0.3 * 440.0 / 680.0, np.array([40.0, 40.0, 9.0])
+
+    def wide(normal, pitch):
+        grid = R.plane_grid(box, (1.0, 2.0, 0.4), normal, 45, 45 * pitch * pixel)
+        return R.staged_traits(maps, N.MR_CONE, 90, 420, dtype, grid.tobytes())[2]
+    assert wide((0.1, -0.05, 1.0), 4.2) > 0.5                            # 130 to 184 columns, 20 rows
+    assert wide((0.0, 0.0, 1.0), 5.5) > 0.3                              # 170 to 241 columns: the wider box

@@ -254,12 +254,21 @@ BLOCK_VOLUME_MIN = 64
 # 64 x 64 x 51 voxels 0.33 and 0.90).
 COARSE_VOXEL_PIXELS = (3.3, 8.0)
 
-# Width of a tile's side (31 sample steps) in detector pixels from which a grid goes to
+# Width of a tile's side (31 sample steps) in detector pixels from which a grid may go to
 # mr_backproject_staged_wide. A view sees a square tile 1 to 1.4 sides wide and a stage takes 76
 # pixels, so from about 64 most views exceed it (25 axial 192^2 slices, side 81: 1739 -> 1003 us);
 # below, the few that do are cheaper through global memory (ten 601^2 slices, side 57: 1243 us,
 # 1316 us with the wide variant).
 WIDE_TILE_PIXELS = 64
+
+# Share of a grid's (tile, view) pairs that only wide boxes hold, from which it does go there. The
+# wide variant reads the other footprints no faster, and those from global memory slower (16-bit
+# rings: up to 1.47 times). A launch within one wave ends with its slowest tile, so up to
+# WIDE_WAVE tiles next to all footprints must be in a stage or a box. Of 3076 random lists (those
+# described at mr_staged_slim_pays) the two conditions take 204: 0.30 to 1.0 times the plain
+# entry's time, 0.54 in the median; by the sample step alone 785 of 1820 were slower.
+WIDE_SHARE, WIDE_FEW_SHARE = 0.4, 0.99
+WIDE_WAVE = 104
 
 # Share of a grid's (tile, view) pairs whose footprint a stage holds, from which the grid may go
 # to mr_backproject_staged_slim. Its four warps hide less of the latency of footprints read from
@@ -449,7 +458,7 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     tile records are uploaded before the stream waits for it (asynchronously from
     page-locked memory with asynchronous=True). band_axis: the orbit's rotation axis, which
     orders the tiles of regular grids by height (_native.plan_tiles). wide: which grids go
-    through mr_backproject_staged_wide (the same result bit for bit; see is_wide), one truth
+    through mr_backproject_staged_wide (the same result bit for bit; see wide_grids), one truth
     value each, or None for none. slim: whether the others go through
     mr_backproject_staged_slim (the same result bit for bit; see slim_pays)."""
     grids = np.ascontiguousarray(grids, dtype=N.GRID_DTYPE)
@@ -518,6 +527,15 @@ def slim_pays(traits, dtype_code):
     """Whether grids of these traits, in one launch, go to mr_backproject_staged_slim."""
     return (all(share >= SLIM_SHARE for _, share, _ in traits)
             and bool(N.load().mr_staged_slim_pays(sum(t[0] for t in traits), dtype_code)))
+
+
+def wide_grids(wide, traits):
+    """Which grids of one list go to mr_backproject_staged_wide: of those that is_wide says (`wide`,
+    one truth value each) the ones whose footprints its boxes hold."""
+    fit = [w and t[2] >= WIDE_SHARE for w, t in zip(wide, traits)]
+    if any(fit) and sum(t[0] for f, t in zip(fit, traits) if f) <= WIDE_WAVE:
+        fit = [f and t[1] + t[2] >= WIDE_FEW_SHARE for f, t in zip(fit, traits)]
+    return fit
 
 
 def is_wide(grid, band_axis, wide_step):
@@ -1448,8 +1466,8 @@ class SliceReconstructor:
 
     def _forms(self, entries):
         """(wide, slim) of backproject_device for a list of _plane_entry's."""
-        wide = [e[1] for e in entries]
-        return wide, slim_pays([e[2] for e in entries if not e[1]], self._dtype_code)
+        wide = wide_grids([e[1] for e in entries], [e[2] for e in entries])
+        return wide, slim_pays([e[2] for w, e in zip(wide, entries) if not w], self._dtype_code)
 
     def _planes(self, requests):
         """One batched launch for many slices -> (flat f32 device tensor, sizes)."""
