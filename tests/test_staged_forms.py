@@ -84,6 +84,17 @@ def test_only_footprints_that_wide_boxes_hold_are_wide(dtype):
     assert chosen((0, 0, 1.0), 6.0, 1, 96) == [False]
 
 
+@pytest.mark.parametrize("dtype", [N.MR_F32, N.MR_BF16])
+def test_few_wide_tiles_share_the_launch_of_the_others(dtype):
+    axial = R.plane_grid(GEOM.volume_box(), (0, 0, 0.5), (0, 0, 1.0), 192)               # 36 tiles
+    other = plane((0.5, 0.4, 0.7), 128)
+    ta, to = traits(axial, dtype), traits(other, dtype)
+    for count in (1, 3, 11):
+        assert R.wide_grids([True] * count + [False], [ta] * count + [to]) == [False] * (count + 1)
+        assert R.wide_grids([True] * count, [ta] * count) == [True] * count
+    assert R.wide_grids([True] * 12 + [False], [ta] * 12 + [to]) == [True] * 12 + [False]
+
+
 def test_traits_argument_checks():
     lib, t = N.load(), (ctypes.c_double * 3)()
     ok = [MAPS.ctypes.data, VIEWS, N.MR_CONE, ROWS, COLS, N.MR_F32, plane((0, 0, 1.0), 64).tobytes(), t]

@@ -270,6 +270,13 @@ WIDE_TILE_PIXELS = 64
 WIDE_SHARE, WIDE_FEW_SHARE = 0.4, 0.99
 WIDE_WAVE = 104
 
+# Busy tiles from which the wide grids of a list get a launch of their own beside the others': the
+# second launch costs its records and a last wave. Axial slices at 2.6 pixels a sample beside
+# others, one launch / two: 36 tiles beside 30 (600 views of 486 x 384, FP32) 478 / 595 us, 216
+# beside 9 (120 views of 1200 x 1000, FP32) 238 / 273, 324 beside 9 there 278 / 297; from 432 tiles
+# on two launches took 0.66 to 0.99 times one's time, whatever was beside them.
+WIDE_SPLIT = 400
+
 # Share of a grid's (tile, view) pairs whose footprint a stage holds, from which the grid may go
 # to mr_backproject_staged_slim. Its four warps hide less of the latency of footprints read from
 # global memory: lists whose grids all have 0.97 or more took 0.70 to 1.0 times the full form's
@@ -531,11 +538,13 @@ def slim_pays(traits, dtype_code):
 
 def wide_grids(wide, traits):
     """Which grids of one list go to mr_backproject_staged_wide: of those that is_wide says (`wide`,
-    one truth value each) the ones whose footprints its boxes hold."""
+    one truth value each) the ones whose footprints its boxes hold, if those are all grids or
+    enough tiles for a launch of their own."""
     fit = [w and t[2] >= WIDE_SHARE for w, t in zip(wide, traits)]
-    if any(fit) and sum(t[0] for f, t in zip(fit, traits) if f) <= WIDE_WAVE:
+    busy = sum(t[0] for f, t in zip(fit, traits) if f)
+    if any(fit) and busy <= WIDE_WAVE:
         fit = [f and t[1] + t[2] >= WIDE_FEW_SHARE for f, t in zip(fit, traits)]
-    return fit
+    return fit if all(fit) or busy >= WIDE_SPLIT else [False] * len(fit)
 
 
 def is_wide(grid, band_axis, wide_step):
