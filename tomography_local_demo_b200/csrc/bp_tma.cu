@@ -69,13 +69,10 @@ enum : int { MODE_WIDE2 = 3, MODE_WIDE3 = 4 };       // beside MODE_STAGED / MOD
 struct __align__(16) ViewRec {
     float4 a, b, c;
 };
-// The producer's copy adds the TMA box origin and count. Wide modes keep detector coordinates
-// (the arithmetic of the global path, bit for bit); `origin` is then the offset that the
-// magic-constant bits of (r0, x0) have.
+// The producer's copy adds the TMA box origin and count.
 struct __align__(16) ViewMeta {
     ViewRec rec;
     int x0, r0, nbox, mode;
-    uint32_t origin;
 };
 
 __device__ __forceinline__ bool in_box_fp64_t(const mr_grid& g, int i, int j) {
@@ -179,7 +176,6 @@ __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g
     const int wcols = mode == MODE_WIDE2 ? StageGeom<T>::W2 : (mode == MODE_WIDE3 ? StageGeom<T>::W3 : W);
     const bool boxes = mode != MODE_GLOBAL && mode != MODE_SKIP;
     const uint32_t maxoff = boxes ? (uint32_t)(nbox * wcols * ST_BOX_H * ESZ - (wcols + 1) * ESZ - ESZ) : 0u;
-    m.origin = (uint32_t)(MAGIC_BITS + r0) * (uint32_t)(wcols * ESZ) + (uint32_t)(MAGIC_BITS + x0) * (uint32_t)ESZ;
     m.rec.a = make_float4(cu.x, cu.y, cu.z, cv.x);
     m.rec.b = make_float4(cv.y, cv.z, aw.x, aw.y);
     m.rec.c = make_float4(aw.z, V.qscale, __uint_as_float(maxoff), __int_as_float(mode));
@@ -229,6 +225,8 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
     uint64_t* empty = full + S;                                                      // S
     float4* partial = reinterpret_cast<float4*>(empty + S);                          // cluster sum: 1024 floats
     __shared__ mr_grid s_g;
+    // wide modes keep detector coordinates (the arithmetic of the global path, bit for bit): the
+    // offset that the magic-constant bits of (r0, x0) have
     __shared__ uint32_t origin_ring[S];
 
     cg::cluster_group cluster = cg::this_cluster();
@@ -332,8 +330,10 @@ bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
                         if (mode == MODE_STAGED) {
                             mbar_arrive_tx(&full[s], (uint32_t)(nbox * BOX_BYTES));
                         } else if (WIDE && (mode == MODE_WIDE2 || mode == MODE_WIDE3)) {
-                            origin_ring[s] = meta_new[l].origin;
-                            mbar_arrive_tx(&full[s], (uint32_t)(nbox * (mode == MODE_WIDE2 ? BOX2_BYTES : BOX3_BYTES)));
+                            const bool w2 = mode == MODE_WIDE2;
+                            origin_ring[s] = (uint32_t)(MAGIC_BITS + meta_new[l].r0) * (uint32_t)((w2 ? W2 : W3) * ESZ) +
+                                             (uint32_t)(MAGIC_BITS + meta_new[l].x0) * (uint32_t)ESZ;
+                            mbar_arrive_tx(&full[s], (uint32_t)(nbox * (w2 ? BOX2_BYTES : BOX3_BYTES)));
                         } else {
                             mbar_arrive(&full[s]);
                         }
@@ -538,10 +538,11 @@ template <int KIND, bool WIDE, bool SLIM, typename T>
 static int launch_staged(const mr_ring* ring, const mr_view* views, const mr_grid* grids,
                          const mr_tile* tiles, int64_t n_tiles, float* out, int* status, cudaStream_t st,
                          const int64_t* n_tiles_dev = nullptr, unsigned int* counter = nullptr) {
-    CUtensorMap map, map2, map3;
+    CUtensorMap map;
     int rc = make_ring_map<T>(ring, StageGeom<T>::W, &map);
-    if (rc == MR_OK) rc = make_ring_map<T>(ring, StageGeom<T>::W2, &map2);
-    if (rc == MR_OK) rc = make_ring_map<T>(ring, StageGeom<T>::W3, &map3);
+    CUtensorMap map2 = map, map3 = map;           // read by WIDE alone
+    if (WIDE && rc == MR_OK) rc = make_ring_map<T>(ring, StageGeom<T>::W2, &map2);
+    if (WIDE && rc == MR_OK) rc = make_ring_map<T>(ring, StageGeom<T>::W3, &map3);
     if (rc != MR_OK) return rc;
     constexpr int S = SLIM ? 2 : StageGeom<T>::STAGES;
     const size_t smem = (size_t)S * StageGeom<T>::W * ST_BOX_H * StageGeom<T>::MAXB * sizeof(T) +
