@@ -31,11 +31,18 @@ namespace mr {
 
 constexpr int GR_THREADS = 256;
 constexpr int GR_PPT = 4;
-constexpr int GR_DI = GR_THREADS / 32;         // row step between a thread's samples
+constexpr int GR_STEP = GR_THREADS / 32;       // lines between a thread's samples
 constexpr int GR_VCH = 128;
 constexpr int GR_TILE = 32;                    // tile edge (samples), as planned by mr_plan_tiles
 
+enum : int { ALONG_J = 0, ALONG_I = 1, PATCHES = 2 };      // a warp's 32 samples
 enum : int { GRAD_ADJOINT = 0, GRAD_GEOM = 1, GRAD_FORWARD = 2 };
+
+// One coordinate of a grid's sample. The roundings are written out: left to the compiler they
+// depend on the code around, and all three kernels use the same coordinates.
+__device__ __forceinline__ float grid_point(const mr_grid& g, int e, int i, int j, int k) {
+    return fmaf((float)k, g.step_k[e], fmaf((float)j, g.step_j[e], fmaf((float)i, g.step_i[e], g.origin[e])));
+}
 
 // Where the footprint of a whole 32 x 32 tile lies in a view: wholly on the detector with a
 // margin of half a pixel (no tap of any lane needs a check), wholly off it (nothing to add),
@@ -71,7 +78,7 @@ __device__ __forceinline__ int tile_footprint(const float* pu, const float* pv, 
 }
 
 template <int KIND, int MODE, typename T>
-__global__ void __launch_bounds__(GR_THREADS, 3)
+__global__ void __launch_bounds__(GR_THREADS, MODE == GRAD_FORWARD ? 4 : 3)
 bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int C, int pitch,
                long long slot_stride, int n_slots, const mr_view* __restrict__ views,
                const mr_grid* __restrict__ grids,
@@ -93,11 +100,48 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
     const mr_grid& g = s_g;
     const bool pts = (g.flags & MR_GRID_POINTS) != 0;
     const int warp = tid >> 5, lane = tid & 31;
-    // a warp takes rows of 32 samples along j, eight rows apart: on a slice j is horizontal, so
-    // a row's taps lie on one or two detector rows and a warp-wide gather or reduction touches
-    // few lines (8 x 4 patches: forward 505, adjoint 830, geometry 497 us where this takes 459,
-    // 705 and 459 with the calls' records; one 512^2 slice, 600 views of 486 x 384)
-    const int tx = lane, ty = warp;
+    int first, nv;                      // slots [first, first + nv)
+    grid_view_range(g.view_begin, g.n_views, n_slots, &first, &nv);
+    // Where a warp's 32 samples lie. On a line, eight lines apart, along the grid direction that
+    // moves less along the detector's rows (j on a slice, i on a volume, whose j is the rotation
+    // axis): its taps then lie on one or two detector rows, and a warp-wide gather or reduction
+    // touches few lines of memory. Where neither direction moves along them (axial slices) and a
+    // sample is wider than 2.5 pixels, in patches of 8 x 4: a line of samples would cover more
+    // memory. Patches / lines along j / this rule:
+    //   512^2 slice, 600 views of 486 x 384, the calls' records included: forward 505 / 459 /
+    //   459 us, adjoint 830 / 705 / 705, geometry 497 / 459 / 459
+    //   160 x 160 x 127 voxels, 180 views of 300 x 200: forward 1.77 / 3.04 / 1.20 ms, adjoint
+    //   4.32 / 8.47 / 2.47 ms, geometry 1.74 / 3.06 / 1.59 ms
+    //   axial 96^2 slice (5 pixels a sample), 300 views of 486 x 384: adjoint 51 / 77 / 51 us
+    int lanes = ALONG_J;
+    if (!pts && nv > 0) {
+        const mr_view& V = views[first];
+        float p[3], row = V.pv[3], col = V.pu[3], vi = 0.f, vj = 0.f, ui = 0.f, uj = 0.f, wi = 0.f, wj = 0.f;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            p[e] = grid_point(g, e, t.i0, t.j0, t.k);
+            row = fmaf(V.pv[e], p[e], row);
+            col = fmaf(V.pu[e], p[e], col);
+            ui = fmaf(V.pu[e], g.step_i[e], ui);
+            uj = fmaf(V.pu[e], g.step_j[e], uj);
+            vi = fmaf(V.pv[e], g.step_i[e], vi);
+            vj = fmaf(V.pv[e], g.step_j[e], vj);
+            wi = fmaf(V.pw[e], g.step_i[e], wi);
+            wj = fmaf(V.pw[e], g.step_j[e], wj);
+        }
+        if (KIND == MR_CONE) {          // d(row) = (d(numerator) - row d(depth)) / depth, and so the column
+            const float w = fmaf(V.pw[0], p[0], fmaf(V.pw[1], p[1], fmaf(V.pw[2], p[2], V.pw[3])));
+            vi = (vi - row / w * wi) / w;
+            vj = (vj - row / w * wj) / w;
+            ui = (ui - col / w * wi) / w;
+            uj = (uj - col / w * wj) / w;
+        }
+        if (fabsf(vi) < 0.7f * fabsf(vj)) lanes = ALONG_I;
+        if (fmaxf(fabsf(vi), fabsf(vj)) < 0.5f && ui * ui + uj * uj > 6.25f) lanes = PATCHES;
+    }
+    const int tx = lanes == ALONG_J ? lane : lanes == ALONG_I ? warp : ((warp & 3) << 3) | (lane & 7);
+    const int ty = lanes == ALONG_J ? warp : lanes == ALONG_I ? lane : ((warp >> 2) << 4) | (lane >> 3);
+    const int dj = lanes == ALONG_I ? GR_STEP : 0, di = lanes == ALONG_J ? GR_STEP : lanes == ALONG_I ? 0 : 4;
 
     float px[GR_PPT], py[GR_PPT], pz[GR_PPT], gp[GR_PPT], acc[GR_PPT];
     long long oidx[GR_PPT];
@@ -113,8 +157,8 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
             ok = j < g.n_j;
             o = g.out_offset + (long long)j * g.out_stride_j;
         } else {
-            i = t.i0 + ty + GR_DI * p;
-            j = t.j0 + tx;
+            i = t.i0 + ty + di * p;
+            j = t.j0 + tx + dj * p;
             ok = i < g.n_i && j < g.n_j;
             o = g.out_offset + (long long)i * g.out_stride_i + (long long)j * g.out_stride_j +
                 (long long)t.k * g.out_stride_k;
@@ -140,9 +184,9 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
             py[p] = g.points[3 * jj + 1];
             pz[p] = g.points[3 * jj + 2];
         } else {
-            px[p] = g.origin[0] + i * g.step_i[0] + j * g.step_j[0] + t.k * g.step_k[0];
-            py[p] = g.origin[1] + i * g.step_i[1] + j * g.step_j[1] + t.k * g.step_k[1];
-            pz[p] = g.origin[2] + i * g.step_i[2] + j * g.step_j[2] + t.k * g.step_k[2];
+            px[p] = grid_point(g, 0, i, j, t.k);
+            py[p] = grid_point(g, 1, i, j, t.k);
+            pz[p] = grid_point(g, 2, i, j, t.k);
         }
     }
     // a warp none of whose samples counts has nothing to do in the view loop
@@ -153,8 +197,6 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
     const float shift = g.cor_shift;
     const float cc = 0.5f * (float)(C - 1), cr = 0.5f * (float)(R - 1);
     float ds = 0.f, dt = 0.f;
-    int first, nv;                      // slots [first, first + nv)
-    grid_view_range(g.view_begin, g.n_views, n_slots, &first, &nv);
     {                                   // this CTA's share of them
         const int b = first + (int)(((long long)nv * crank) / csize);
         const int e = first + (int)(((long long)nv * (crank + 1)) / csize);
@@ -305,7 +347,7 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
 #pragma unroll
         for (int p = 0; p < GR_PPT; ++p) {
             const bool ok = pts ? (t.j0 + tid + GR_THREADS * p < g.n_j)
-                                : (t.i0 + ty + GR_DI * p < g.n_i && t.j0 + tx < g.n_j);
+                                : (t.i0 + ty + di * p < g.n_i && t.j0 + tx + dj * p < g.n_j);
             if (ok) {
                 const float val = live[p] ? acc[p] * g.scale : 0.f;
                 gring[oidx[p]] = g.accumulate ? gring[oidx[p]] + val : val;
@@ -333,14 +375,15 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
 template <int KIND, int MODE, typename T>
 static int launch_grad(const mr_ring* ring, float* gring, const mr_view* views, const mr_grid* grids,
                        const mr_tile* tiles, int64_t n_tiles, const float* gout, double* dgeom, cudaStream_t st) {
-    // CTAs per tile: enough for about five waves of three CTAs an SM, at most 8 (portable
-    // cluster). Tiles differ in how many of their samples count, so short CTAs even out (256
-    // tiles: 8 CTAs each 551, 4 each 698 us for the geometry gradient)
+    // CTAs per tile: enough for eight an SM, at most 8 (portable cluster). Tiles differ in how
+    // many of their samples count, so short CTAs even out (256 tiles: 8 CTAs each 551, 4 each
+    // 698 us for the geometry gradient); more than that cost more than they even out (864 tiles
+    // of a 96 x 96 x 76 volume, 180 views: 376 us forward with one, 405 with two, 468 with four)
     int dev = 0, sms = 148;
     MR_CUDA_TRY(cudaGetDevice(&dev));
     MR_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int cl = 1;
-    while (cl < 8 && n_tiles * cl < 16LL * sms) cl *= 2;
+    while (cl < 8 && n_tiles * cl < 8LL * sms) cl *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GR_THREADS);
     cfg.stream = st;
