@@ -422,9 +422,10 @@ int mr_volume_select(const float* vol, int64_t n, const int64_t* ranks_host, int
                      uint32_t kmin, uint32_t kmax, void* ws, float* values_dev, void* stream);
 
 /* The same for ranks near quantiles q_lo <= q_hi of the non-zero voxels, with one read of the
- * volume: mr_volume_tails brackets both quantiles by a sample and collects the voxels at and
- * beyond the brackets into ws (16-byte aligned here); stats_host (host) = {nonzero, nan, voxels
- * of the lower tail, voxels of the upper tail}; the call waits for the stream.
+ * volume: mr_volume_tails brackets both quantiles by a sample, counts the voxels at and beyond
+ * the brackets and collects those beyond into ws (16-byte aligned here); stats_host (host) =
+ * {nonzero, nan, voxels of the lower tail, voxels of the upper tail}, the tails with those equal
+ * to the bracket; the call waits for the stream.
  * mr_volume_tail_select: as mr_volume_select, from the stats and the tails in ws;
  * MR_ERR_UNSUPPORTED when a rank lies in neither tail or its tail is too large to be kept
  * (many equal voxels): use mr_volume_stats and mr_volume_select then. */
@@ -432,6 +433,11 @@ int mr_volume_tails(const float* vol, int64_t n, double q_lo, double q_hi, void*
                     uint64_t* stats_host, void* stream);
 int mr_volume_tail_select(const int64_t* ranks_host, int32_t n_ranks, const uint64_t* stats_host,
                           void* ws, float* values_dev, void* stream);
+
+/* The same where a tail is too large only for the voxels that equal its bracket: those are counted,
+ * not kept, so any number of them will do. The call waits for the stream. */
+int mr_volume_tail_select_equal(const int64_t* ranks_host, int32_t n_ranks, const uint64_t* stats_host,
+                                void* ws, float* values_dev, void* stream);
 
 /* hist_dev[b] (device, bins uint64, overwritten) = the number of non-zero, non-NaN voxels
  * whose FP64 value clipped to [lo, hi] falls in bin b of numpy.histogram(..., bins,

@@ -99,6 +99,7 @@ SIGNATURES = {
     "mr_volume_select": (ctypes.c_int, [_P, _I64, _P, _I32, ctypes.c_uint32, ctypes.c_uint32, _P, _P, _P]),
     "mr_volume_tails": (ctypes.c_int, [_P, _I64, ctypes.c_double, ctypes.c_double, _P, _P, _P]),
     "mr_volume_tail_select": (ctypes.c_int, [_P, _I32, _P, _P, _P, _P]),
+    "mr_volume_tail_select_equal": (ctypes.c_int, [_P, _I32, _P, _P, _P, _P]),
     "mr_volume_histogram": (ctypes.c_int, [_P, _I64, _P, _I32, ctypes.c_double, ctypes.c_double, _P, _P]),
     "mr_rotate_f32": (ctypes.c_int, [_P, _P, _I32, _I32, _I32, ctypes.c_double, _P]),
     "mr_gaussian_axis_f32": (ctypes.c_int, [_P, _P, _I32, _I32, _I32, _I32, _I32, _P, _I32, _P]),

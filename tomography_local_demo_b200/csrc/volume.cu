@@ -9,7 +9,8 @@
 //   mr_volume_histogram  numpy's uniform-bin histogram of the FP64-clipped values
 // and, for the two percentiles of the clip, one pass in the place of stats and select:
 //   mr_volume_tails      brackets both percentiles by a sample, then counts the voxels and
-//                        collects those outside the brackets (a few per mille)
+//                        collects those outside the brackets (a few per mille; those equal to
+//                        a bracket, which may be any number, are only counted)
 //   mr_volume_tail_select  exact order statistics among the collected ones
 // The percentile interpolation and the Otsu arithmetic over the bins stay on the host,
 // in FP64 as the reference computes them.
@@ -34,7 +35,7 @@ constexpr int VOL_DIGITS = 1 << VOL_RADIX;
 constexpr uint32_t VOL_NONE = 0xffffffffu;
 constexpr unsigned FULL = 0xffffffffu;
 
-constexpr int TAIL_CAP = 1 << 21;               // voxels kept of each tail
+constexpr int TAIL_CAP = 1 << 22;               // voxels kept of each tail
 constexpr int TAIL_SAMPLE = 16384;
 
 // Device workspace of the entry points (the first part zeroed by mr_volume_stats, the tails'
@@ -47,8 +48,9 @@ struct VolState {
     unsigned long long rank[VOL_MAX_RANKS]; // rank left inside the current prefix
     unsigned long long hist[VOL_MAX_RANKS][VOL_DIGITS];
     unsigned long long t_nonzero, t_nan, t_count[2];    // mr_volume_tails: voxels != 0, NaNs, size of each tail
+    unsigned long long t_beyond[2];         // those that are not equal to the edge
     float t_edge[2];                        // tail 0: x <= t_edge[0]; tail 1: x >= t_edge[1]
-    __align__(16) float tail[2][TAIL_CAP];
+    __align__(16) float tail[2][TAIL_CAP];  // the voxels beyond the edges
 };
 
 // Order-preserving map of a float onto an unsigned key (negatives reversed below positives).
@@ -259,15 +261,23 @@ vol_histogram_kernel(const float* __restrict__ v, long long n, const double* __r
     __shared__ unsigned int h[VOL_MAX_BINS + 1];            // [bins]: zeros, NaNs, lanes past the end
     __shared__ float lb[VOL_MAX_BINS + 1];
     __shared__ int s_bin_lo, s_bin_hi;
-    for (int i = threadIdx.x; i <= bins; i += blockDim.x) h[i] = 0u;
-    for (int i = threadIdx.x; i <= bins; i += blockDim.x) lb[i] = __double2float_ru(edges[i]);
-    if (threadIdx.x == 0) {
-        // bins of the clip bounds themselves (lo, hi inside [edges[0], edges[bins]])
-        int a = 0, b = bins - 1;
-        while (a < bins - 1 && lo >= edges[a + 1]) ++a;
-        while (b > 0 && hi < edges[b]) --b;
-        s_bin_lo = a;
-        s_bin_hi = b;
+    if (threadIdx.x == 0) s_bin_lo = s_bin_hi = 0;
+    __syncthreads();
+    // the bins of the clip bounds themselves: how many inner edges lie at or below them (a search
+    // by one thread took 100 us at 2048 bins where both lie in the middle, a volume of one value)
+    int below_lo = 0, below_hi = 0;
+    for (int i = threadIdx.x; i <= bins; i += blockDim.x) {
+        const double e = edges[i];
+        h[i] = 0u;
+        lb[i] = __double2float_ru(e);
+        below_lo += i > 0 && i < bins && e <= lo;
+        below_hi += i > 0 && i < bins && e <= hi;
+    }
+    below_lo = __reduce_add_sync(FULL, below_lo);
+    below_hi = __reduce_add_sync(FULL, below_hi);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&s_bin_lo, below_lo);
+        atomicAdd(&s_bin_hi, below_hi);
     }
     __syncthreads();
     const float lo_up = __double2float_ru(lo), hi_dn = __double2float_rd(hi);
@@ -307,8 +317,23 @@ vol_histogram_kernel(const float* __restrict__ v, long long n, const double* __r
 // instead of four. 134 M voxels: 30 us sample, 106 us pass (82 us at the copy rate), 34 us
 // selection, against 124 us stats and 728 us of select passes. A sample of 32768 made the
 // tails 0.6 times as large and took 45 us itself.
+// Voxels equal to a bracket are counted and not collected: where one value is frequent (clipped,
+// masked or whole-numbered volumes) they may be most of the volume (512^3, the whole threshold, by
+// the select passes / by tails that hold them / by these: one value 0.71 / 6.05 / 0.71 ms, two
+// values 2.06 / 4.68 / 0.75 ms, half the voxels clipped 1.87 / 3.61 / 0.70 ms).
 constexpr int TAIL_THREADS = 1024;
 constexpr int TAIL_OWN = TAIL_SAMPLE / TAIL_THREADS;
+
+// One count more, by the lanes that call it together: as one where their digits are all the same
+// (the leading digits of any volume, all four of a volume of one value, which otherwise took 70 us
+// longer).
+__device__ __forceinline__ void sample_add(unsigned int* bin, uint32_t digit) {
+    const unsigned active = __activemask();
+    int same;
+    __match_all_sync(active, digit, &same);
+    if (!same) atomicAdd(bin, 1u);
+    else if ((int)(threadIdx.x & 31) == __ffs(active) - 1) atomicAdd(bin, (unsigned)__popc(active));
+}
 
 // One block; each thread holds 16 sampled keys, and both ranks are found by four rounds of
 // 8-bit digits.
@@ -365,8 +390,8 @@ vol_tail_sample_kernel(const float* __restrict__ v, long long n, double q_lo, do
         for (int u = 0; u < TAIL_OWN; ++u) {
             if (key[u] == VOL_NONE) continue;
             const uint32_t d = (key[u] >> shift) & 255u;
-            if ((key[u] & above) == p0) atomicAdd(&hist[0][d], 1u);
-            if (p1 != p0 && (key[u] & above) == p1) atomicAdd(&hist[1][d], 1u);
+            if ((key[u] & above) == p0) sample_add(&hist[0][d], d);
+            if (p1 != p0 && (key[u] & above) == p1) sample_add(&hist[1][d], d);
         }
         __syncthreads();
         if (tid < 64) {                                     // a warp per rank, 8 bins a lane
@@ -396,22 +421,23 @@ vol_tail_sample_kernel(const float* __restrict__ v, long long n, double q_lo, do
     if (tid < 2) st->t_edge[tid] = key_value(s_prefix[tid]);
 }
 
-constexpr int TAIL_LIST = 1024;                  // voxels of each tail a block collects before it hands them on
+constexpr int TAIL_LIST = 2048;                  // voxels of each tail a block collects before it hands them on
 
 __global__ void __launch_bounds__(VOL_THREADS) vol_tail_kernel(const float* __restrict__ v, long long n, VolState* st) {
     __shared__ float list[2][TAIL_LIST];
-    __shared__ unsigned int s_n[2], s_at[2];
+    __shared__ unsigned int s_n[2], s_sum[4];               // s_sum: as t_nonzero, t_nan, t_count
+    __shared__ unsigned long long first[2];
     const float low = st->t_edge[0], high = st->t_edge[1];
     if (threadIdx.x < 2) s_n[threadIdx.x] = 0u;
+    if (threadIdx.x < 4) s_sum[threadIdx.x] = 0u;
     __syncthreads();
-    unsigned int nz = 0;
-    unsigned int nan = 0;
+    unsigned int nz = 0, nan = 0, size[2] = {0u, 0u};       // < 2^32: a block sees fewer than 2^32 voxels
     auto put = [&](int t, float x) {
         const unsigned int at = atomicAdd(&s_n[t], 1u);
         if (at < TAIL_LIST) {
             list[t][at] = x;
         } else {                                            // the block's list is full: straight to the tail
-            const unsigned long long o = atomicAdd(&st->t_count[t], 1ull);
+            const unsigned long long o = atomicAdd(&st->t_beyond[t], 1ull);
             if (o < TAIL_CAP) st->tail[t][o] = x;
         }
     };
@@ -420,34 +446,41 @@ __global__ void __launch_bounds__(VOL_THREADS) vol_tail_kernel(const float* __re
         nz += some;
         if (some && !(x > low && x < high)) {               // a tail's voxel, or NaN
             nan += x != x;
-            if (x <= low) put(0, x);
-            if (x >= high) put(1, x);
+            if (x <= low) {
+                ++size[0];
+                if (x < low) put(0, x);
+            }
+            if (x >= high) {
+                ++size[1];
+                if (x > high) put(1, x);
+            }
         }
     });
-    nz = __reduce_add_sync(FULL, nz);                       // < 2^32: a thread sees fewer than 2^27 voxels
-    nan = __reduce_add_sync(FULL, nan);
+    const unsigned int sum[4] = {__reduce_add_sync(FULL, nz), __reduce_add_sync(FULL, nan),
+                                 __reduce_add_sync(FULL, size[0]), __reduce_add_sync(FULL, size[1])};
     if ((threadIdx.x & 31) == 0) {
-        if (nz) atomicAdd(&st->t_nonzero, (unsigned long long)nz);
-        if (nan) atomicAdd(&st->t_nan, (unsigned long long)nan);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (sum[i]) atomicAdd(&s_sum[i], sum[i]);
     }
     __syncthreads();
+    if (threadIdx.x < 4 && s_sum[threadIdx.x])              // one of each a block: they all meet at one address
+        atomicAdd(&st->t_nonzero + threadIdx.x, (unsigned long long)s_sum[threadIdx.x]);
     for (int t = 0; t < 2; ++t) {
         const unsigned int k = min(s_n[t], (unsigned int)TAIL_LIST);
-        __shared__ unsigned long long first[2];
-        if (threadIdx.x == 0 && k) first[t] = atomicAdd(&st->t_count[t], (unsigned long long)k);
+        if (threadIdx.x == 0 && k) first[t] = atomicAdd(&st->t_beyond[t], (unsigned long long)k);
         __syncthreads();
         for (unsigned int i = threadIdx.x; i < k; i += VOL_THREADS)
             if (first[t] + i < TAIL_CAP) st->tail[t][first[t] + i] = list[t][i];
     }
 }
 
-// Exact order statistics among the collected tails: a cluster of 8 CTAs per rank, three rounds
+// Exact order statistics of the tails, of which a run of voxels equals the edge: a cluster of 8 CTAs per rank, three rounds
 // of 11, 11 and 10 bit digits, the digit histograms added through distributed shared memory.
 constexpr int TSEL_CLUSTER = 8;
 struct TailRanks {
     long long rank[VOL_MAX_RANKS];              // within its tail
     int tail[VOL_MAX_RANKS];
-    long long n[VOL_MAX_RANKS];
 };
 __global__ void __launch_bounds__(TAIL_THREADS)
 vol_tail_select_kernel(const VolState* __restrict__ st, TailRanks tr, float* __restrict__ out) {
@@ -458,12 +491,20 @@ vol_tail_select_kernel(const VolState* __restrict__ st, TailRanks tr, float* __r
     cg::cluster_group cluster = cg::this_cluster();
     const int crank = (int)cluster.block_rank(), j = blockIdx.x / TSEL_CLUSTER;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float* __restrict__ x = st->tail[tr.tail[j]];
-    const long long n = tr.n[j], per = ((n + TSEL_CLUSTER - 1) / TSEL_CLUSTER + 3) / 4 * 4;
+    const int t = tr.tail[j];
+    const float* __restrict__ x = st->tail[t];
+    const long long n = (long long)st->t_beyond[t], equal = (long long)st->t_count[t] - n;
+    // the edge's own run: the lower tail's last voxels, the upper one's first
+    const long long rank = t == 0 ? tr.rank[j] : tr.rank[j] - equal;
+    if (t == 0 ? rank >= n : rank < 0) {                    // the same for the whole cluster
+        if (crank == 0 && tid == 0) out[j] = st->t_edge[t];
+        return;
+    }
+    const long long per = ((n + TSEL_CLUSTER - 1) / TSEL_CLUSTER + 3) / 4 * 4;
     const long long b = min(n, per * crank), e = min(n, b + per);
     if (tid == 0) {
         s_prefix = 0u;
-        s_rank = (unsigned long long)tr.rank[j];
+        s_rank = (unsigned long long)rank;
     }
     for (int shift = 21; shift >= 0; shift = shift == 21 ? 10 : (shift == 10 ? 0 : -1)) {
         const int width = shift == 0 ? 10 : 11;
@@ -580,7 +621,7 @@ extern "C" int mr_volume_tails(const float* vol, int64_t n, double q_lo, double 
     int blocks = 0;
     const int rc = mr::vol_grid(&blocks);
     if (rc != MR_OK) return rc;
-    MR_CUDA_TRY(cudaMemsetAsync(&s->t_nonzero, 0, 4 * sizeof(uint64_t), st));
+    MR_CUDA_TRY(cudaMemsetAsync(&s->t_nonzero, 0, 6 * sizeof(uint64_t), st));
     if (n > 0) {
         mr::vol_tail_sample_kernel<<<1, mr::TAIL_THREADS, 0, st>>>(vol, (long long)n, q_lo, q_hi, s);
         mr::vol_tail_kernel<<<blocks, mr::VOL_THREADS, 0, st>>>(vol, (long long)n, s);
@@ -591,25 +632,25 @@ extern "C" int mr_volume_tails(const float* vol, int64_t n, double q_lo, double 
     return MR_OK;
 }
 
-extern "C" int mr_volume_tail_select(const int64_t* ranks, int32_t n_ranks, const uint64_t* stats_host, void* ws,
-                                     float* values_dev, void* stream) {
-    if (!ranks || !stats_host || !ws || !values_dev || n_ranks < 1 || n_ranks > mr::VOL_MAX_RANKS) return MR_ERR_INVALID;
-    if ((uintptr_t)ws & 15u) return MR_ERR_INVALID;
+// beyond: how many voxels lie beyond each edge, at most the tails' places; null: the tails of
+// stats_host, edges included, have to be no larger than those.
+static int tail_select(const int64_t* ranks, int32_t n_ranks, const uint64_t* stats_host, const uint64_t* beyond,
+                       void* ws, float* values_dev, void* stream) {
     const uint64_t live = stats_host[0] - stats_host[1];
     mr::TailRanks tr = {};
     for (int j = 0; j < n_ranks; ++j) {
         if (ranks[j] < 0 || (uint64_t)ranks[j] >= live) return MR_ERR_INVALID;
         const uint64_t r = (uint64_t)ranks[j];
-        if (stats_host[2] <= mr::TAIL_CAP && r < stats_host[2]) {
+        const uint64_t* kept = beyond ? beyond : stats_host + 2;
+        if (kept[0] <= mr::TAIL_CAP && r < stats_host[2]) {
             tr.tail[j] = 0;
             tr.rank[j] = (long long)r;
-        } else if (stats_host[3] <= mr::TAIL_CAP && r >= live - stats_host[3]) {
+        } else if (kept[1] <= mr::TAIL_CAP && r >= live - stats_host[3]) {
             tr.tail[j] = 1;
             tr.rank[j] = (long long)(r - (live - stats_host[3]));
         } else {
             return MR_ERR_UNSUPPORTED;
         }
-        tr.n[j] = (long long)stats_host[2 + tr.tail[j]];
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_ranks * mr::TSEL_CLUSTER));
@@ -625,6 +666,27 @@ extern "C" int mr_volume_tail_select(const int64_t* ranks, int32_t n_ranks, cons
     MR_CUDA_TRY(cudaLaunchKernelEx(&cfg, mr::vol_tail_select_kernel, (const mr::VolState*)ws, tr, values_dev));
     MR_CUDA_TRY(cudaGetLastError());
     return MR_OK;
+}
+
+static bool tail_args(const int64_t* ranks, int32_t n_ranks, const uint64_t* stats_host, void* ws, float* values_dev) {
+    return ranks && stats_host && ws && values_dev && n_ranks >= 1 && n_ranks <= mr::VOL_MAX_RANKS &&
+           !((uintptr_t)ws & 15u);
+}
+
+extern "C" int mr_volume_tail_select(const int64_t* ranks, int32_t n_ranks, const uint64_t* stats_host, void* ws,
+                                     float* values_dev, void* stream) {
+    if (!tail_args(ranks, n_ranks, stats_host, ws, values_dev)) return MR_ERR_INVALID;
+    return tail_select(ranks, n_ranks, stats_host, nullptr, ws, values_dev, stream);
+}
+
+extern "C" int mr_volume_tail_select_equal(const int64_t* ranks, int32_t n_ranks, const uint64_t* stats_host, void* ws,
+                                           float* values_dev, void* stream) {
+    if (!tail_args(ranks, n_ranks, stats_host, ws, values_dev)) return MR_ERR_INVALID;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    uint64_t beyond[2];
+    MR_CUDA_TRY(cudaMemcpyAsync(beyond, static_cast<mr::VolState*>(ws)->t_beyond, sizeof(beyond), cudaMemcpyDeviceToHost, st));
+    MR_CUDA_TRY(cudaStreamSynchronize(st));
+    return tail_select(ranks, n_ranks, stats_host, beyond, ws, values_dev, stream);
 }
 
 extern "C" int mr_volume_histogram(const float* vol, int64_t n, const double* edges_dev, int32_t bins,
