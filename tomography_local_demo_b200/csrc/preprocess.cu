@@ -218,6 +218,14 @@ static size_t gauss_lines_smem(int K, int TO) {
     return ((size_t)(TO + GS_TAPS * nb) * (LP + 1) + 2 * (size_t)GS_TAPS * nb) * sizeof(float);
 }
 
+// Most outputs of 4 lines that gauss_lines_smem<4> leaves room for (a multiple of GS_RUN; may be
+// negative).
+static int gauss_few_outputs(int K, size_t limit) {
+    const long long span = GS_TAPS * (long long)((2 * (long long)K + GS_TAPS) / GS_TAPS);
+    const long long room = ((long long)(limit / sizeof(float)) - 2 * span) / 5 - span;
+    return (int)(room / GS_RUN * GS_RUN);
+}
+
 template <int L, int LP>
 static int launch_gauss_lines(const float* in, float* out, int R, int A, int C, int axis, int pad, const float* taps,
                               int K, int TO, cudaStream_t st) {
@@ -262,13 +270,19 @@ extern "C" int mr_gaussian_axis_f32(const float* in, float* out, int32_t rows, i
     const int n = axis == 0 ? rows : cols;
     constexpr size_t kSmemMax = 200 * 1024;
     // whole lines per block (16 lines: every input staged about twice, the periodic
-    // extension) where they fit, else 8 lines x 512 outputs
+    // extension) where they fit, else 8 lines x 512 outputs, else 4 lines and as many outputs as
+    // fit (more than 1750 taps a side: axes of 3500 to 7000 pixels; one view of 3600 x 3504, both
+    // axes, 6.0 ms, 115.9 by the loop without staging, which longer axes are left to)
+    const int few = mr::gauss_few_outputs(K, kSmemMax);
     const int whole = (n + mr::GS_RUN - 1) / mr::GS_RUN * mr::GS_RUN;
     if (K <= n + 2 * pad && mr::gauss_lines_smem<18>(K, whole) <= kSmemMax) {
         const int rc = mr::launch_gauss_lines<16, 18>(in, out, rows, k, cols, axis, pad, taps, K, whole, st);
         if (rc != MR_OK) return rc;
     } else if (K <= n + 2 * pad && mr::gauss_lines_smem<10>(K, 512) <= kSmemMax) {
         const int rc = mr::launch_gauss_lines<8, 10>(in, out, rows, k, cols, axis, pad, taps, K, 512, st);
+        if (rc != MR_OK) return rc;
+    } else if (K <= n + 2 * pad && few >= 256) {
+        const int rc = mr::launch_gauss_lines<4, 4>(in, out, rows, k, cols, axis, pad, taps, K, few < whole ? few : whole, st);
         if (rc != MR_OK) return rc;
     } else {
         const dim3 block(128);
