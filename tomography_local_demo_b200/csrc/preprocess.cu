@@ -15,15 +15,17 @@ namespace mr {
 // Where an output samples its view, and with what weights, is the same in every view: a thread
 // forms both once for RT_VIEWS views and has the taps of all of them in flight, where a thread of
 // one output waited for its four loads alone (486 x 384, 0.3 degrees: 600 views 483 -> 227 us,
-// 64 views 57 -> 32 us, 8 views 12 -> 10 us, one view 8 us as before; 16 views of 1944 x 1536
-// 209 -> 94 us; the same outputs). A read and a write of the 600 views take 137 us; what is left
-// is latency and issue (63 %) of the four loads an output.
+// 64 views 57 -> 32 us, 8 views 12 -> 10 us; 1944 x 1536: 64 views 816 -> 352 us, 8 views 106 ->
+// 46, 2 views 29 -> 25; the same outputs). One view has nothing to share and keeps a kernel of its
+// own (1944 x 1536: 18.3 us, 23.2 with the other). A read and a write of the 600 views take 137
+// us; what is left is latency and issue (63 %) of the four loads an output.
 constexpr int RT_VIEWS = 8;
+template <int VIEWS>
 __global__ void __launch_bounds__(128) rotate_kernel(const float* __restrict__ in, float* __restrict__ out, int R,
                                                      int A, int C, float ct, float st) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y;
-    const int a0 = blockIdx.z * RT_VIEWS;
+    const int a0 = blockIdx.z * VIEWS;
     if (c >= C) return;
     const float rr = (float)r - 0.5f * (float)(R - 1);
     const float cc = (float)c - 0.5f * (float)(C - 1);
@@ -60,8 +62,8 @@ __global__ void __launch_bounds__(128) rotate_kernel(const float* __restrict__ i
             o[(long long)(a + v) * C] = acc;
         }
     };
-    const int n = min(RT_VIEWS, A - a0);
-    if (n == RT_VIEWS) views(0, std::integral_constant<int, RT_VIEWS>{});
+    const int n = min(VIEWS, A - a0);
+    if (n == VIEWS) views(0, std::integral_constant<int, VIEWS>{});
     else
         for (int a = 0; a < n; ++a) views(a, std::integral_constant<int, 1>{});
 }
@@ -250,9 +252,10 @@ extern "C" int mr_rotate_f32(const float* in, float* out, int32_t rows, int32_t 
     if (k == 0) return MR_OK;
     const double t = degrees * 3.14159265358979323846 / 180.0;
     const dim3 block(128);
-    const dim3 grid((cols + 127) / 128, rows, (k + mr::RT_VIEWS - 1) / mr::RT_VIEWS);
+    const int views = k == 1 ? 1 : mr::RT_VIEWS;
+    const dim3 grid((cols + 127) / 128, rows, (k + views - 1) / views);
     if (k > 65535 || rows > 65535) return MR_ERR_INVALID;
-    mr::rotate_kernel<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(
+    (views == 1 ? mr::rotate_kernel<1> : mr::rotate_kernel<mr::RT_VIEWS>)<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(
         in, out, rows, k, cols, (float)cos(t), (float)sin(t));
     MR_CUDA_TRY(cudaGetLastError());
     return MR_OK;
