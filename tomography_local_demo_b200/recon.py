@@ -373,8 +373,11 @@ _STAGING_LOCK = threading.Lock()
 
 
 def _staging(device):
-    """The record staging ring of `device` (created on first use)."""
+    """The record staging ring of `device` (created on first use), which without an index is the
+    current one: the ring's events belong to the device of their first record."""
     key = torch.device(device).index
+    if key is None:
+        key = torch.cuda.current_device()
     with _STAGING_LOCK:
         if key not in _STAGING:
             _STAGING[key] = _RecordStaging()
