@@ -469,7 +469,7 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     page-locked memory with asynchronous=True). band_axis: the orbit's rotation axis, which
     orders the tiles of regular grids by height (_native.plan_tiles). wide: which grids go
     through mr_backproject_staged_wide (the same result bit for bit; see wide_grids), one truth
-    value each, or None for none. slim: whether the others go through
+    value each (those of point lists do not count), or None for none. slim: whether the others go through
     mr_backproject_staged_slim (the same result bit for bit; see slim_pays)."""
     grids = np.ascontiguousarray(grids, dtype=N.GRID_DTYPE)
     is_pts = (grids["flags"] & N.MR_GRID_POINTS) != 0
@@ -477,6 +477,7 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
         backproject_device(ring, views_dev, grids[is_pts], out, stream, device, timer, "plain", wait=wait,
                            asynchronous=asynchronous)
         wait = None
+        wide = None if wide is None else [w for w, p in zip(wide, is_pts) if not p]
         grids = grids[~is_pts]
         is_pts = is_pts[~is_pts]
     all_wide = wide is not None and kernel == "staged" and len(grids) > 0 and not is_pts.any() and all(wide)
