@@ -180,18 +180,44 @@ def marching_cubes(vol, iso, origin=(0.0, 0.0, 0.0), spacing=1.0):
         if min(nx, ny, nz) < 2:
             return (torch.zeros((0, 3), dtype=torch.float32, device=dev),
                     torch.zeros((0, 3), dtype=torch.int64, device=dev))
-        ws = torch.empty(int(lib.mr_mesh_workspace_bytes(nx, ny, nz)), dtype=torch.uint8, device=dev)
+        org = (ctypes.c_double * 3)(*[float(x) for x in origin])
+        try:
+            ws = torch.empty(int(lib.mr_mesh_workspace_bytes(nx, ny, nz)), dtype=torch.uint8, device=dev)
+        except torch.OutOfMemoryError:
+            return _cells_mesh(lib, t, float(iso), org, float(spacing), stream)
         totals = (ctypes.c_int64 * 3)()
         N.check(lib.mr_mesh_plan(v(t.data_ptr()), nx, ny, nz, float(iso), v(ws.data_ptr()), totals,
                                  v(stream.cuda_stream)), "mr_mesh_plan")
         n_tri, n_vert = int(totals[0]), int(totals[1])
         points = torch.empty((n_vert, 3), dtype=torch.float32, device=dev)
         faces = torch.empty((n_tri, 3), dtype=torch.int64, device=dev)
-        org = (ctypes.c_double * 3)(*[float(x) for x in origin])
         N.check(lib.mr_mesh_emit(v(t.data_ptr()), nx, ny, nz, float(iso), org, float(spacing), v(ws.data_ptr()),
                                  totals, v(points.data_ptr()) if n_vert else None,
                                  v(faces.data_ptr()) if n_tri else None, v(stream.cuda_stream)), "mr_mesh_emit")
         return points, faces
+
+
+def _cells_mesh(lib, t, iso, org, spacing, stream):
+    """The same mesh for a volume that leaves no room for mr_mesh_plan's workspace (0.3 times its
+    own size, more where it is thin along z): two passes over its cells (mr_mc_count, mr_mc_emit),
+    which need memory for the surface alone, and a sort that merges the copies of each vertex by
+    its grid edge. 320 x 320 x 301 voxels, 0.5 M triangles: 0.98 ms, by marching_cubes 0.16."""
+    nx, ny, nz = t.shape
+    v, dev = ctypes_void, t.device
+    counts = torch.empty(int(lib.mr_mc_blocks(nx, ny, nz)), dtype=torch.int32, device=dev)
+    N.check(lib.mr_mc_count(v(t.data_ptr()), nx, ny, nz, iso, v(counts.data_ptr()), v(stream.cuda_stream)), "mr_mc_count")
+    c64 = counts.to(torch.int64)
+    offsets = torch.cumsum(c64, 0) - c64
+    total = int(c64.sum())
+    edges = torch.empty(3 * total, dtype=torch.int64, device=dev)
+    pos = torch.empty((3 * total, 3), dtype=torch.float32, device=dev)
+    N.check(lib.mr_mc_emit(v(t.data_ptr()), nx, ny, nz, iso, org, spacing, v(offsets.data_ptr()), total,
+                           v(edges.data_ptr()) if total else None, v(pos.data_ptr()) if total else None,
+                           v(stream.cuda_stream)), "mr_mc_emit")
+    uniq, inv = torch.unique(edges, return_inverse=True)
+    points = torch.empty((len(uniq), 3), dtype=torch.float32, device=dev)
+    points[inv] = pos                           # every copy of a vertex holds the same value
+    return points, inv.view(-1, 3)
 
 
 def _components(faces, n_points):
