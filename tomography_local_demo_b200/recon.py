@@ -263,8 +263,8 @@ WIDE_TILE_PIXELS = 64
 
 # Share of a grid's (tile, view) pairs that only wide boxes hold, from which it does go there. The
 # wide variant reads the other footprints no faster, and those from global memory slower (16-bit
-# rings: up to 1.47 times). A launch within one wave ends with its slowest tile, so up to
-# WIDE_WAVE tiles next to all footprints must be in a stage or a box. Of 3076 random lists (those
+# rings: up to 1.47 times). A launch within one wave (104 clusters of the full form) ends with its
+# slowest tile, so up to WIDE_WAVE tiles next to all footprints must be in a stage or a box. Of 3076 random lists (those
 # described at mr_staged_slim_pays) the two conditions take 204: 0.30 to 1.0 times the plain
 # entry's time, 0.54 in the median; by the sample step alone 785 of 1820 were slower.
 WIDE_SHARE, WIDE_FEW_SHARE = 0.4, 0.99
@@ -281,8 +281,12 @@ WIDE_SPLIT = 400
 # to mr_backproject_staged_slim. Its four warps hide less of the latency of footprints read from
 # global memory: lists whose grids all have 0.97 or more took 0.70 to 1.0 times the full form's
 # time, from 0.95 on up to 1.1, without the condition up to 1.7 (the 3076 lists described at the
-# count of tiles that pays, mr_staged_slim_pays).
+# count of tiles that pays, mr_staged_slim_pays). Lists of many tiles ride out some grids with less
+# (their slowest tiles end beside others): 16-bit rings from 1200 busy tiles and 0.75 of all pairs
+# on 0.73 to 0.96 times, FP32 from 2000 and 0.985 on 0.91 to 0.99 (0.95: up to 1.05; below 1200
+# tiles up to 1.15).
 SLIM_SHARE = 0.97
+SLIM_MANY = {False: (1200, 0.75), True: (2000, 0.985)}       # FP32 ring: busy tiles, share of all pairs
 
 
 def _device(device=None):
@@ -536,8 +540,17 @@ def staged_traits(maps, kind_code, rows, cols, dtype_code, grid):
 
 def slim_pays(traits, dtype_code):
     """Whether grids of these traits, in one launch, go to mr_backproject_staged_slim."""
-    return (all(share >= SLIM_SHARE for _, share, _ in traits)
-            and bool(N.load().mr_staged_slim_pays(sum(t[0] for t in traits), dtype_code)))
+    fp32 = dtype_code == N.MR_F32
+    busy, staged, least = 0, 0.0, 1.0
+    for tiles, share, _ in traits:
+        busy += tiles
+        staged += tiles * share
+        least = min(least, share)
+    if busy <= WIDE_WAVE:
+        return False
+    many, part = SLIM_MANY[fp32]
+    return ((least >= SLIM_SHARE or busy >= many and staged >= part * busy)
+            and bool(N.load().mr_staged_slim_pays(busy, dtype_code)))
 
 
 def wide_grids(wide, traits):
@@ -1479,8 +1492,11 @@ class SliceReconstructor:
 
     def _forms(self, entries):
         """(wide, slim) of backproject_device for a list of _plane_entry's."""
-        wide = wide_grids([e[1] for e in entries], [e[2] for e in entries])
-        return wide, slim_pays([e[2] for w, e in zip(wide, entries) if not w], self._dtype_code)
+        traits = [e[2] for e in entries]
+        if True not in [e[1] for e in entries]:
+            return None, slim_pays(traits, self._dtype_code)
+        wide = wide_grids([e[1] for e in entries], traits)
+        return wide, slim_pays([t for w, t in zip(wide, traits) if not w], self._dtype_code)
 
     def _planes(self, requests):
         """One batched launch for many slices -> (flat f32 device tensor, sizes)."""
