@@ -1373,7 +1373,7 @@ class SliceReconstructor:
         waits only for its own chunk's filter, so the reconstruction overlaps the transfer
         of the later chunks (same scale; FP32 partial sums added in view order). Called with the
         device and the reconstruction stream current. wide, slim: see backproject_device (slim
-        None: found out here)."""
+        None: found out here, for one large grid)."""
         stream = self.stream
         grids["scale"] = np.pi / n if n else 0.0
         marks = [(se, e) for se, e in self._chunk_marks if 0 < se < n]
@@ -1389,7 +1389,9 @@ class SliceReconstructor:
                                           self._status, coarse)
             return
         if slim is None and regular and self.bp_kernel == "staged":
-            slim = slim_pays([self._traits(g.tobytes()) for g in grids], self._dtype_code)
+            # the traits cost 7 us a grid, which small volumes would wait for
+            large = len(grids) == 1 and math.prod(grids[0][k].item() for k in ("n_i", "n_j", "n_k")) >= 400 * 1024
+            slim = large and slim_pays([self._traits(grids[0].tobytes())], self._dtype_code)
         if marks and regular and self.bp_kernel == "staged":
             bounds = [0] + [se for se, _ in marks] + [n]
             events = [e for _, e in marks] + [event]
