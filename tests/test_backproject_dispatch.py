@@ -22,10 +22,11 @@ class Pointer:
         pass
 
 
-@pytest.mark.parametrize("slim", [False, True])
-@pytest.mark.parametrize("kinds", ["www", "www.", "pww", "wpw.", "p.w.pw", "pp", "p.", "..", "pwpw"])
+@pytest.mark.parametrize("slim", [False, True, None])
+@pytest.mark.parametrize("kinds", ["www", "www.", "pww", "wpw.", "p.w.pw", "pp", "p.", "..", "pwpw", "s.", "ss", "pswp.s", "sw"])
 def test_entries(monkeypatch, kinds, slim):
-    """kinds: w = wide, p = points, . = another regular grid; grid k has k + 1 tiles."""
+    """kinds: w = wide, p = points, s = slim where that is said grid by grid (slim None), . = another
+    regular grid; grid k has k + 1 tiles."""
     box = np.array([40.0, 40.0, 40.0])
     grids = np.zeros(len(kinds), N.GRID_DTYPE)
     for k, kind in enumerate(kinds):
@@ -46,8 +47,13 @@ def test_entries(monkeypatch, kinds, slim):
     native.load = lambda: lib
     monkeypatch.setattr(R, "N", native)
     monkeypatch.setattr(R, "_struct_tensor", lambda *a: Pointer())
-    R.backproject_device(None, Pointer(), grids, Pointer(), Pointer(), None, wide=[k == "w" for k in kinds], slim=slim)
-    rest = "mr_backproject_staged_slim" if slim else "mr_backproject_staged"
-    want = {n: sum(k + 1 for k, kind in enumerate(kinds) if kind == c)
-            for c, n in (("p", "mr_backproject"), ("w", "mr_backproject_staged_wide"), (".", rest))}
+    R.backproject_device(None, Pointer(), grids, Pointer(), Pointer(), None, wide=[k == "w" for k in kinds],
+                         slim=[k == "s" for k in kinds] if slim is None else slim)
+    forms = {"p": "mr_backproject", "w": "mr_backproject_staged_wide", "s": "mr_backproject_staged_slim",
+             ".": "mr_backproject_staged"}
+    if slim is not None:
+        forms["s"] = forms["."] = forms["s" if slim else "."]
+    want = dict.fromkeys(forms.values(), 0)
+    for k, kind in enumerate(kinds):
+        want[forms[kind]] += k + 1
     assert dict(calls) == {n: t for n, t in want.items() if t} and len(calls) == len(dict(calls))

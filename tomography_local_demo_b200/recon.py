@@ -283,10 +283,17 @@ WIDE_SPLIT = 400
 # time, from 0.95 on up to 1.1, without the condition up to 1.7 (the 3076 lists described at the
 # count of tiles that pays, mr_staged_slim_pays). Lists of many tiles ride out some grids with less
 # (their slowest tiles end beside others): 16-bit rings from 1200 busy tiles and 0.75 of all pairs
-# on 0.73 to 0.96 times, FP32 from 2000 and 0.985 on 0.91 to 0.99 (0.95: up to 1.05; below 1200
-# tiles up to 1.15).
+# on 0.73 to 0.96 times, FP32 from 2000 and 0.975 on 0.82 to 0.98, one of 14 lists 1.02 (below, a
+# hundredth of the pairs costs four of the time: 0.95 up to 1.08, 0.9 up to 1.10).
 SLIM_SHARE = 0.97
-SLIM_MANY = {False: (1200, 0.75), True: (2000, 0.985)}       # FP32 ring: busy tiles, share of all pairs
+SLIM_MANY = {False: (1200, 0.75), True: (2000, 0.975)}       # FP32 ring: busy tiles, share of all pairs
+
+# Busy tiles of the grids with SLIM_SHARE from which they get a launch of their own beside the
+# others', where one launch of the four-warp form does not pay (FP32 ring, 160 full-resolution views,
+# one launch of the eight-warp form / two: 1207 tiles beside 144 646 / 607 us, 3456 beside 1728
+# 1970 / 1990, 5871 beside 576 1558 / 1465; 33789 beside 4611, 400 views, 36.6 / 33.1 ms, where
+# one of the four-warp form took 34.3).
+SLIM_SPLIT = 5000
 
 
 def _device(device=None):
@@ -473,24 +480,27 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     page-locked memory with asynchronous=True). band_axis: the orbit's rotation axis, which
     orders the tiles of regular grids by height (_native.plan_tiles). wide: which grids go
     through mr_backproject_staged_wide (the same result bit for bit; see wide_grids), one truth
-    value each (those of point lists do not count), or None for none. slim: whether the others go through
-    mr_backproject_staged_slim (the same result bit for bit; see slim_pays)."""
+    value each (those of point lists do not count), or None for none. slim: which of the others go
+    through mr_backproject_staged_slim (the same result bit for bit; see slim_grids), one truth
+    value for all or one each."""
     grids = np.ascontiguousarray(grids, dtype=N.GRID_DTYPE)
     is_pts = (grids["flags"] & N.MR_GRID_POINTS) != 0
+    per_grid = [slim] * len(grids) if slim is True or slim is False else list(slim)
+    forms = ["wide" if w else "slim" if f else "" for w, f in zip(wide or [False] * len(grids), per_grid)]
     if kernel == "staged" and is_pts.any() and not is_pts.all():
         backproject_device(ring, views_dev, grids[is_pts], out, stream, device, timer, "plain", wait=wait,
                            asynchronous=asynchronous)
         wait = None
-        wide = None if wide is None else [w for w, p in zip(wide, is_pts) if not p]
+        forms = [f for f, p in zip(forms, is_pts) if not p]
         grids = grids[~is_pts]
         is_pts = is_pts[~is_pts]
-    all_wide = wide is not None and kernel == "staged" and len(grids) > 0 and not is_pts.any() and all(wide)
-    if not all_wide and wide is not None and kernel == "staged" and not is_pts.any() and any(wide):
-        w = np.asarray(wide, dtype=bool)
-        for part, flag in ((grids[w], [True] * int(w.sum())), (grids[~w], None)):
-            backproject_device(ring, views_dev, part, out, stream, device, timer, kernel, status, wait, asynchronous,
-                               band_axis, flag, slim)
-            wait = None
+    if kernel == "staged" and not is_pts.any() and len(set(forms)) > 1:
+        for form in ("wide", "slim", ""):
+            part = grids[[f == form for f in forms]]
+            if len(part):
+                backproject_device(ring, views_dev, part, out, stream, device, timer, kernel, status, wait, asynchronous,
+                                   band_axis, [True] * len(part) if form == "wide" else None, form == "slim")
+                wait = None
         return
     tiles = N.plan_tiles(grids, band_axis)
     if len(tiles) == 0:
@@ -509,7 +519,7 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     name = "mr_backproject_staged" if staged else "mr_backproject"
     ev0 = timer.start(stream) if timer is not None else None
     if staged:
-        fn = staged_entry(lib, all_wide, slim)
+        fn = staged_entry(lib, forms[0])
         st = fn(ring, v(views_dev.data_ptr()), v(g_ptr), v(t_ptr), len(tiles), v(out.data_ptr()),
                 v(status.data_ptr()) if status is not None else None, v(stream.cuda_stream))
     else:
@@ -522,11 +532,10 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     recs.record_stream(stream)
 
 
-def staged_entry(lib, wide, slim):
-    """The library's entry of that form of the staged back-projection."""
-    if wide:
-        return lib.mr_backproject_staged_wide
-    return lib.mr_backproject_staged_slim if slim else lib.mr_backproject_staged
+def staged_entry(lib, form):
+    """The library's entry of a form of the staged back-projection ("wide", "slim" or "")."""
+    return {"wide": lib.mr_backproject_staged_wide, "slim": lib.mr_backproject_staged_slim,
+            "": lib.mr_backproject_staged}[form]
 
 
 def staged_traits(maps, kind_code, rows, cols, dtype_code, grid):
@@ -551,6 +560,15 @@ def slim_pays(traits, dtype_code):
     many, part = SLIM_MANY[fp32]
     return ((least >= SLIM_SHARE or busy >= many and staged >= part * busy)
             and bool(N.load().mr_staged_slim_pays(busy, dtype_code)))
+
+
+def slim_grids(traits, dtype_code):
+    """Which grids of these traits go to mr_backproject_staged_slim: all (True), none (False) or one
+    truth value each."""
+    if slim_pays(traits, dtype_code):
+        return True
+    fit = [t[1] >= SLIM_SHARE for t in traits]
+    return fit if sum([t[0] for f, t in zip(fit, traits) if f]) >= SLIM_SPLIT else False
 
 
 def wide_grids(wide, traits):
@@ -1405,7 +1423,8 @@ class SliceReconstructor:
             if len(tiles) == 0:
                 return
             lib = N.load()
-            launch = staged_entry(lib, wide and all(wide), slim and not (wide and any(wide)))
+            form = "wide" if wide and all(wide) else "slim" if slim is True and not wide else ""
+            launch = staged_entry(lib, form)
             v = ctypes_void
             with torch.cuda.device(self.device), torch.cuda.stream(stream):
                 # one upload for all ranges and the tiles; launch i reads its own G records
@@ -1431,7 +1450,7 @@ class SliceReconstructor:
         backproject_device(self._ring_c, self._views_dev, grids, out, stream, self.device,
                            self.kernel_timer, self.bp_kernel, self._status, wait=event,
                            asynchronous=not self._chunk_marks, band_axis=self._band_axis, wide=wide,
-                           slim=bool(slim))
+                           slim=slim if slim is not None else False)
 
     def reconstruct_points_tensor(self, pts, cor_shift=None):
         """Device variant of reconstruct_points: pts (M, 3) -> f32 tensor [M]."""
@@ -1496,9 +1515,17 @@ class SliceReconstructor:
         """(wide, slim) of backproject_device for a list of _plane_entry's."""
         traits = [e[2] for e in entries]
         if True not in [e[1] for e in entries]:
-            return None, slim_pays(traits, self._dtype_code)
+            return None, slim_grids(traits, self._dtype_code)
         wide = wide_grids([e[1] for e in entries], traits)
-        return wide, slim_pays([t for w, t in zip(wide, traits) if not w], self._dtype_code)
+        if all(wide):
+            return wide, False
+        if not any(wide):
+            return None, slim_grids(traits, self._dtype_code)
+        rest = slim_grids([t for w, t in zip(wide, traits) if not w], self._dtype_code)
+        if rest is True or rest is False:
+            return wide, rest
+        rest = iter(rest)
+        return wide, [not w and next(rest) for w in wide]
 
     def _planes(self, requests):
         """One batched launch for many slices -> (flat f32 device tensor, sizes)."""
@@ -1896,7 +1923,7 @@ class ScanReplay:
             return
         lib, v = N.load(), ctypes_void
         base = self.recs.data_ptr()
-        fn = staged_entry(lib, False, self._slim) if rec.bp_kernel == "staged" else lib.mr_backproject
+        fn = staged_entry(lib, "slim" if self._slim else "") if rec.bp_kernel == "staged" else lib.mr_backproject
         name = "mr_backproject_staged" if rec.bp_kernel == "staged" else "mr_backproject"
         args = [rec._ring_c, v(rec._views_dev.data_ptr()), v(base + self._g_off), v(base + self._t_off),
                 self.n_tiles, v(self.out.data_ptr())]
