@@ -23,7 +23,7 @@ class Pointer:
 
 
 @pytest.mark.parametrize("slim", [False, True, None])
-@pytest.mark.parametrize("kinds", ["www", "www.", "pww", "wpw.", "p.w.pw", "pp", "p.", "..", "pwpw", "s.", "ss", "pswp.s", "sw"])
+@pytest.mark.parametrize("kinds", ["www", "ww", "www.", "pww", "wpw.", "p.w.pw", "pp", "p.", "..", "pwpw", "s.", "ss", "pswp.s", "sw"])
 def test_entries(monkeypatch, kinds, slim):
     """kinds: w = wide, p = points, s = slim where that is said grid by grid (slim None), . = another
     regular grid; grid k has k + 1 tiles."""
@@ -47,7 +47,8 @@ def test_entries(monkeypatch, kinds, slim):
     native.load = lambda: lib
     monkeypatch.setattr(R, "N", native)
     monkeypatch.setattr(R, "_struct_tensor", lambda *a: Pointer())
-    R.backproject_device(None, Pointer(), grids, Pointer(), Pointer(), None, wide=[k == "w" for k in kinds],
+    R.backproject_device(None, Pointer(), grids, Pointer(), Pointer(), None,
+                         wide=True if kinds == "www" else [k == "w" for k in kinds],
                          slim=[k == "s" for k in kinds] if slim is None else slim)
     forms = {"p": "mr_backproject", "w": "mr_backproject_staged_wide", "s": "mr_backproject_staged_slim",
              ".": "mr_backproject_staged"}

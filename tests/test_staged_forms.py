@@ -68,9 +68,9 @@ def test_launches_of_the_four_warp_form():
     # some grids that are staged in part, in a list of many tiles and in a shorter one
     part, whole = (300, 0.5, 0.0), (300, 1.0, 0.0)
     assert [R.slim_pays([part] * a + [whole] * b, N.MR_BF16) for a, b in ((1, 2), (2, 6), (5, 3))] == [False, True, False]
-    assert [R.slim_pays([(60, 0.7, 0.0)] + [whole] * b, N.MR_F32) for b in (3, 6, 8)] == [False, False, True]
+    assert [R.slim_pays([(60, 0.7, 0.0)] + [whole] * b, N.MR_F32) for b in (3, 9, 10)] == [False, False, True]
     assert R.slim_grids([whole, part], N.MR_F32) is False and R.slim_grids([whole] * 2, N.MR_F32) is True
-    assert R.slim_grids([part, part, (6000, 1.0, 0.0)], N.MR_F32) == [False, False, True]
+    assert R.slim_grids([part] * 3 + [(6000, 1.0, 0.0)], N.MR_F32) == [False] * 3 + [True]
 
 
 @pytest.mark.parametrize("dtype", [N.MR_F32, N.MR_BF16])

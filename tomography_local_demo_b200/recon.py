@@ -283,10 +283,10 @@ WIDE_SPLIT = 400
 # time, from 0.95 on up to 1.1, without the condition up to 1.7 (the 3076 lists described at the
 # count of tiles that pays, mr_staged_slim_pays). Lists of many tiles ride out some grids with less
 # (their slowest tiles end beside others): 16-bit rings from 1200 busy tiles and 0.75 of all pairs
-# on 0.73 to 0.96 times, FP32 from 2000 and 0.975 on 0.82 to 0.98, one of 14 lists 1.02 (below, a
-# hundredth of the pairs costs four of the time: 0.95 up to 1.08, 0.9 up to 1.10).
+# on 0.73 to 0.96 times, FP32 from 3000 and 0.95 on 0.90 to 1.0 (a hundredth of the pairs costs two
+# to four of the time: 0.9 up to 1.04, and at 2000 tiles 0.95 up to 1.08).
 SLIM_SHARE = 0.97
-SLIM_MANY = {False: (1200, 0.75), True: (2000, 0.975)}       # FP32 ring: busy tiles, share of all pairs
+SLIM_MANY = {False: (1200, 0.75), True: (3000, 0.95)}       # FP32 ring: busy tiles, share of all pairs
 
 # Busy tiles of the grids with SLIM_SHARE from which they get a launch of their own beside the
 # others', where one launch of the four-warp form does not pay (FP32 ring, 160 full-resolution views,
@@ -479,14 +479,18 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
     tile records are uploaded before the stream waits for it (asynchronously from
     page-locked memory with asynchronous=True). band_axis: the orbit's rotation axis, which
     orders the tiles of regular grids by height (_native.plan_tiles). wide: which grids go
-    through mr_backproject_staged_wide (the same result bit for bit; see wide_grids), one truth
-    value each (those of point lists do not count), or None for none. slim: which of the others go
+    through mr_backproject_staged_wide (the same result bit for bit; see wide_grids): one truth
+    value each (those of point lists do not count), True for all or None for none. slim: which of the others go
     through mr_backproject_staged_slim (the same result bit for bit; see slim_grids), one truth
     value for all or one each."""
     grids = np.ascontiguousarray(grids, dtype=N.GRID_DTYPE)
     is_pts = (grids["flags"] & N.MR_GRID_POINTS) != 0
-    per_grid = [slim] * len(grids) if slim is True or slim is False else list(slim)
-    forms = ["wide" if w else "slim" if f else "" for w, f in zip(wide or [False] * len(grids), per_grid)]
+    one = wide is True or wide is None and (slim is True or slim is False)
+    if one:
+        forms = ["wide" if wide else "slim" if slim else ""] * len(grids)
+    else:
+        per_grid = [slim] * len(grids) if slim is True or slim is False else slim
+        forms = ["wide" if w else "slim" if f else "" for w, f in zip(wide or [False] * len(grids), per_grid)]
     if kernel == "staged" and is_pts.any() and not is_pts.all():
         backproject_device(ring, views_dev, grids[is_pts], out, stream, device, timer, "plain", wait=wait,
                            asynchronous=asynchronous)
@@ -494,12 +498,12 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
         forms = [f for f, p in zip(forms, is_pts) if not p]
         grids = grids[~is_pts]
         is_pts = is_pts[~is_pts]
-    if kernel == "staged" and not is_pts.any() and len(set(forms)) > 1:
+    if not one and kernel == "staged" and not is_pts.any() and len(set(forms)) > 1:
         for form in ("wide", "slim", ""):
             part = grids[[f == form for f in forms]]
             if len(part):
                 backproject_device(ring, views_dev, part, out, stream, device, timer, kernel, status, wait, asynchronous,
-                                   band_axis, [True] * len(part) if form == "wide" else None, form == "slim")
+                                   band_axis, True if form == "wide" else None, form == "slim")
                 wait = None
         return
     tiles = N.plan_tiles(grids, band_axis)
@@ -567,8 +571,9 @@ def slim_grids(traits, dtype_code):
     truth value each."""
     if slim_pays(traits, dtype_code):
         return True
-    fit = [t[1] >= SLIM_SHARE for t in traits]
-    return fit if sum([t[0] for f, t in zip(fit, traits) if f]) >= SLIM_SPLIT else False
+    if sum([t[0] for t in traits if t[1] >= SLIM_SHARE]) < SLIM_SPLIT:
+        return False
+    return [t[1] >= SLIM_SHARE for t in traits]
 
 
 def wide_grids(wide, traits):
@@ -576,10 +581,10 @@ def wide_grids(wide, traits):
     one truth value each) the ones whose footprints its boxes hold, if those are all grids or
     enough tiles for a launch of their own."""
     fit = [w and t[2] >= WIDE_SHARE for w, t in zip(wide, traits)]
-    busy = sum(t[0] for f, t in zip(fit, traits) if f)
-    if any(fit) and busy <= WIDE_WAVE:
+    busy = sum([t[0] for t in traits]) if False not in fit else sum([t[0] for f, t in zip(fit, traits) if f])
+    if busy <= WIDE_WAVE:
         fit = [f and t[1] + t[2] >= WIDE_FEW_SHARE for f, t in zip(fit, traits)]
-    return fit if all(fit) or busy >= WIDE_SPLIT else [False] * len(fit)
+    return fit if False not in fit or busy >= WIDE_SPLIT else [False] * len(fit)
 
 
 def is_wide(grid, band_axis, wide_step):
@@ -1423,7 +1428,7 @@ class SliceReconstructor:
             if len(tiles) == 0:
                 return
             lib = N.load()
-            form = "wide" if wide and all(wide) else "slim" if slim is True and not wide else ""
+            form = "wide" if wide is True else "slim" if slim is True and wide is None else ""
             launch = staged_entry(lib, form)
             v = ctypes_void
             with torch.cuda.device(self.device), torch.cuda.stream(stream):
@@ -1488,9 +1493,10 @@ class SliceReconstructor:
         return staged_traits(self._maps_all, self._kind_code, self.geom.rows, self.geom.cols, self._dtype_code, grid)
 
     def _plane_entry(self, origin, normal, n, size, zoom, center, shift):
-        """(record bytes, wide, traits) of plane_grid for this reconstructor's box, memoised on the
-        request's parameters (the FP64 plane set-up is pure; a repeated request skips it on the
-        host). wide: see is_wide; traits: see staged_traits."""
+        """[record bytes, wide, tiles, traits] of plane_grid for this reconstructor's box, memoised on
+        the request's parameters (the FP64 plane set-up is pure; a repeated request skips it on the
+        host). wide: see is_wide; tiles: how many; traits: see staged_traits, found when a list
+        first depends on them (None before)."""
         scale = (n, None if size is None else float(size), float(zoom), float(shift))
         try:
             key = (tuple(map(float, origin)), tuple(map(float, normal)),
@@ -1502,8 +1508,7 @@ class SliceReconstructor:
         entry = cache.get(key)
         if entry is None:
             rec = plane_grid(self.box, origin, normal, n, size, zoom, center, shift)
-            raw = rec.tobytes()
-            entry = (raw, is_wide(rec, self._band_axis, self._wide_step), self._traits(raw))
+            entry = [rec.tobytes(), is_wide(rec, self._band_axis, self._wide_step), (-(-n // 32)) ** 2, None]
             cache[key] = entry
             if len(cache) > 256:
                 cache.popitem(last=False)
@@ -1511,21 +1516,31 @@ class SliceReconstructor:
             cache.move_to_end(key)
         return entry
 
+    def _entry_traits(self, entries):
+        traits = [e[3] for e in entries]
+        if None in traits:
+            for e in entries:
+                if e[3] is None:
+                    e[3] = self._traits(e[0])
+            traits = [e[3] for e in entries]
+        return traits
+
     def _forms(self, entries):
         """(wide, slim) of backproject_device for a list of _plane_entry's."""
-        traits = [e[2] for e in entries]
-        if True not in [e[1] for e in entries]:
-            return None, slim_grids(traits, self._dtype_code)
-        wide = wide_grids([e[1] for e in entries], traits)
-        if all(wide):
-            return wide, False
-        if not any(wide):
-            return None, slim_grids(traits, self._dtype_code)
-        rest = slim_grids([t for w, t in zip(wide, traits) if not w], self._dtype_code)
-        if rest is True or rest is False:
-            return wide, rest
-        rest = iter(rest)
-        return wide, [not w and next(rest) for w in wide]
+        wide = [e[1] for e in entries]
+        if True in wide:
+            wide = wide_grids(wide, self._entry_traits(entries))
+            if False not in wide:
+                return True, False
+        rest = [e for w, e in zip(wide, entries) if not w]
+        slim = (sum([e[2] for e in rest]) > WIDE_WAVE
+                and slim_grids(self._entry_traits(rest), self._dtype_code))
+        if True not in wide:
+            return None, slim
+        if slim is True or slim is False:
+            return wide, slim
+        slim = iter(slim)
+        return wide, [not w and next(slim) for w in wide]
 
     def _planes(self, requests):
         """One batched launch for many slices -> (flat f32 device tensor, sizes)."""
@@ -1879,7 +1894,7 @@ class ScanReplay:
         grids["out_offset"] = offsets
         grids["n_views"] = k
         grids["scale"] = np.pi / k
-        self._slim = slim_pays([e[2] for e in entries], rec._dtype_code)
+        self._slim = slim_pays(rec._entry_traits(entries), rec._dtype_code)
         tiles = N.plan_tiles(grids, rec._band_axis)
         self.stream = torch.cuda.Stream(dev)
         rec.reset()
