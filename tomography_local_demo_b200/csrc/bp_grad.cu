@@ -77,6 +77,8 @@ __device__ __forceinline__ int tile_footprint(const float* pu, const float* pv, 
     return cmin > 0.5f && rmin > 0.5f && cmax < (float)C - 1.5f && rmax < (float)R - 1.5f ? FOOT_INSIDE : FOOT_EDGE;
 }
 
+// Four CTAs an SM for the forward kernel (64 registers, up to 88 bytes spilled), three for the others:
+// by 68 grids, forward with three 1.06 times, geometry with four 1.10 times the time.
 template <int KIND, int MODE, typename T>
 __global__ void __launch_bounds__(GR_THREADS, MODE == GRAD_FORWARD ? 4 : 3)
 bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int C, int pitch,
@@ -108,8 +110,9 @@ bp_grad_kernel(const T* __restrict__ ring, float* __restrict__ gring, int R, int
     // touches few lines of memory. Where neither direction moves along them (axial slices) and a
     // sample is wider than 2.5 pixels, in patches of 8 x 4: a line of samples would cover more
     // memory. Patches / lines along j / this rule:
-    //   512^2 slice, 600 views of 486 x 384, the calls' records included: forward 505 / 459 /
-    //   459 us, adjoint 830 / 705 / 705, geometry 497 / 459 / 459
+    //   512^2 slice, 600 views of 486 x 384, whole calls (the kernels alone by this rule: 364 to
+    //   403, 510 and 336 to 350 us): forward 505 / 459 / 459 us, adjoint 830 / 705 / 705, geometry
+    //   497 / 459 / 459
     //   160 x 160 x 127 voxels, 180 views of 300 x 200: forward 1.77 / 3.04 / 1.20 ms, adjoint
     //   4.32 / 8.47 / 2.47 ms, geometry 1.74 / 3.06 / 1.59 ms
     //   axial 96^2 slice (5 pixels a sample), 300 views of 486 x 384: adjoint 51 / 77 / 51 us

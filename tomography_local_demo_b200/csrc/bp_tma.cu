@@ -8,14 +8,14 @@
 //     detector are zero-filled by the TMA unit, which is exactly the reference's
 //     "bilinear taps outside [0,R)x[0,C) contribute 0";
 //   * a warp-specialised ring of stages: one producer warp computes footprints and issues
-//     the TMA loads, eight consumer warps back-project; full/empty mbarriers (bounded
-//     waits) are the only synchronisation inside the view loop;
+//     the TMA loads, eight (four in the slim form) consumer warps back-project; full/empty
+//     mbarriers (bounded waits) are the only synchronisation inside the view loop;
 //   * the consumer loop is predicate-free: floor via a round-down FMA against a magic
 //     constant (FMA pipe only), one unsigned clamp for memory safety, four LDS, lerps;
 //   * footprints that miss the detector entirely are skipped (exactly zero), and the
 //     rare footprints larger than a stage fall back to predicated global loads.
-// Each warp covers compact 8 (j) x 4 (i) sample patches so its LDS gathers touch a small
-// 2D patch (few bank conflicts) for any plane orientation.
+// Each warp covers 16 (j) x 2 (i) sample patches, which keep its taps on distinct banks for most
+// plane orientations.
 #include <cooperative_groups.h>
 #include <cmath>
 
@@ -28,9 +28,10 @@ namespace mr {
 constexpr int ST_TI = 32, ST_TJ = 32;        // tile (samples) - same tiling as bp.cu
 // Consumer warps of a 32 x 32 tile, and one producer warp. SLIM: half the warps with twice the
 // samples each, which share a view's records and waits and run interleaved, and two stages, so
-// that five CTAs fit an SM (four of FP32); for launches with tiles to fill them (slim_pays).
+// that five CTAs fit an SM (four of FP32); for launches of many staged tiles (slim_pays).
 // Three 512^2 slices, 600 views, BF16: 508 -> 462 us; one 1024^2 slice 990 -> 876 us; ten 601^2
-// slices of 160 full-resolution views, FP32: 1242 -> 1217 us. Three stages and four CTAs an SM:
+// slices of 160 full-resolution views, FP32: 0.94 to 1.09 times, by how many of their footprints
+// are staged. Three stages and four CTAs an SM:
 // 459, 819 and 1290 us; a ring of footprint-sized pieces in the place of fixed stages: 518 and
 // 910 us (its bookkeeping is in the producer's path, which the consumers wait for).
 template <bool SLIM> struct Shape {
@@ -183,15 +184,15 @@ __device__ __forceinline__ ViewMeta view_meta(const mr_view& V, const mr_grid& g
     return m;
 }
 
-// Warp-specialised: warps 0..7 consume (256 threads x 4 samples = one 32x32 tile), warp 8
-// produces. Stage s carries the TMA data and its ViewMeta; full[s] (1 arrival + TMA bytes)
+// Warp-specialised: the first warps consume (eight of 4 samples a thread or, SLIM, four of 8: one
+// 32 x 32 tile), the last one produces. Stage s carries the TMA data and its ViewMeta; full[s] (1 arrival + TMA bytes)
 // and empty[s] (one arrival per consumer warp) hand it back and forth. No CTA-wide barrier
 // in the view loop, so consumer warps may run up to S views apart.
 // A thread-block cluster of ST_CLUSTER CTAs shares one tile: CTA rank r back-projects the
 // r-th quarter of the views and rank 0 sums the partials from the others' shared memory
 // (DSMEM) in rank order - deterministic, no atomics, no scratch - and writes the tile.
-// Three CTAs fit an SM (shared memory); the launch bound says so, or ptxas aims at four and
-// spills the FP32 variant to fit its registers.
+// Three CTAs fit an SM (shared memory; SLIM: five, four of FP32); the launch bound says so, or
+// ptxas aims at four and spills the FP32 variant to fit its registers. SLIM spills 4 bytes.
 template <int KIND, bool WIDE, bool SLIM, typename T>
 __global__ void __launch_bounds__(Shape<SLIM>::THREADS, Shape<SLIM>::CTAS)
 bp_staged_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap2,

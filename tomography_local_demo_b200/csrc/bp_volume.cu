@@ -16,8 +16,9 @@
 // voxels, BF16 ring, 16.9 -> 5.9 ms (1360 G updates/s); FP32 ring, whose tile footprints
 // there did not fit a stage, 52.5 -> 6.2 ms; 400 x 400 x 317 voxels 57.3 -> 22.4 ms; views
 // that are not aligned with j, 16.9 -> 8.1 ms. What bounds it: four shared-memory loads a
-// sample (8 samples a clock and SM at most, 2270 G/s) beside 13 issue slots. Two CTAs an SM
-// with all the registers they want measured 6.5 ms.
+// sample (8 samples a clock and SM at most, 2270 G/s) beside 13 issue slots. Three CTAs an SM
+// leave 72 registers (the cone variants spill 48 to 52 bytes); two CTAs with all the registers
+// they want measured 6.5 ms.
 #include <cooperative_groups.h>
 
 #include "bp_stage.cuh"
