@@ -538,8 +538,8 @@ def backproject_device(ring, views_dev, grids, out, stream, device, timer=None, 
 
 def staged_entry(lib, form):
     """The library's entry of a form of the staged back-projection ("wide", "slim" or "")."""
-    return {"wide": lib.mr_backproject_staged_wide, "slim": lib.mr_backproject_staged_slim,
-            "": lib.mr_backproject_staged}[form]
+    return (lib.mr_backproject_staged_slim if form == "slim" else
+            lib.mr_backproject_staged_wide if form == "wide" else lib.mr_backproject_staged)
 
 
 def staged_traits(maps, kind_code, rows, cols, dtype_code, grid):
@@ -553,17 +553,14 @@ def staged_traits(maps, kind_code, rows, cols, dtype_code, grid):
 
 def slim_pays(traits, dtype_code):
     """Whether grids of these traits, in one launch, go to mr_backproject_staged_slim."""
-    fp32 = dtype_code == N.MR_F32
-    busy, staged, least = 0, 0.0, 1.0
-    for tiles, share, _ in traits:
-        busy += tiles
-        staged += tiles * share
-        least = min(least, share)
+    busy = sum([t[0] for t in traits])
     if busy <= WIDE_WAVE:
         return False
-    many, part = SLIM_MANY[fp32]
-    return ((least >= SLIM_SHARE or busy >= many and staged >= part * busy)
-            and bool(N.load().mr_staged_slim_pays(busy, dtype_code)))
+    if min([t[1] for t in traits]) < SLIM_SHARE:
+        many, part = SLIM_MANY[dtype_code == N.MR_F32]
+        if busy < many or sum([t[0] * t[1] for t in traits]) < part * busy:
+            return False
+    return bool(N.load().mr_staged_slim_pays(busy, dtype_code))
 
 
 def slim_grids(traits, dtype_code):
